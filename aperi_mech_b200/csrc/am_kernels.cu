@@ -15,6 +15,8 @@
 #include <math_constants.h>
 #include <stdlib.h>
 
+#include <algorithm>
+
 #include "am_kernels.cuh"
 #include "am_math.cuh"
 
@@ -758,10 +760,6 @@ __global__ void __launch_bounds__(256) k_hex6_patch_dx(const int32_t* __restrict
 // sum applies -1/512 once. Per element this is about half the arithmetic of
 // evaluating the 24 shape-function derivatives at every Gauss point.
 // ---------------------------------------------------------------------------
-// Gauss points unrolled two at a time: full unrolling raises the FP32 kernel to
-// 168 registers and spills the FP64 one; two keeps both in registers.
-constexpr int kHexGpUnroll = 2;
-
 __host__ __device__ constexpr int hex_node_of_corner(int q) { return q ^ ((q >> 1) & 1); }
 
 // v[K] <- sum_a S_K(a) v[a] (corner-bit order): C_0 in v[0], C_j in v[1 << j].
@@ -849,101 +847,306 @@ __device__ __forceinline__ void hex_conn(const GaussBlockDev& b, int64_t e, int3
     nd[0] = c0.x, nd[1] = c0.y, nd[2] = c0.z, nd[3] = c0.w, nd[4] = c1.x, nd[5] = c1.y, nd[6] = c1.z, nd[7] = c1.w;
 }
 
-// The FP32 kernel is held to 128 registers (four 128-thread blocks per SM); the
-// FP64 one keeps its ~250 registers (forcing three blocks per SM spills and was
-// slower on B200) and runs in 64-thread blocks.
-template <typename T, int MAT>
-__global__ void __launch_bounds__(sizeof(T) == 8 ? 64 : 128, sizeof(T) == 8 ? 1 : 4) k_hex8_force(GaussBlockDev b, const double4* __restrict__ X4,
-                                                         const double4* __restrict__ U4,
-                                                         vec4_t<T>* __restrict__ slots, int* status) {
-    const int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (e >= b.num_elems) return;
-    int32_t nd[8];
-    hex_conn(b, e, nd);
-    T X[3][8], U[3][8];
-    hex_load_rel(X4, nd, X);
-    pdl_trigger();
-    pdl_wait();
-    hex_load_rel<T, true>(U4, nd, U);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        hex_butterfly(X[i]);
-        hex_butterfly(U[i]);
-        hex_scale_coeffs(X[i]);
-        hex_scale_coeffs(U[i]);
-    }
-    double lam, mu;
-    element_lame(b, e, lam, mu);
-    T R[3][8];
+// ---------------------------------------------------------------------------
+// Hex8, total formulation: four lanes per element, a warp per eight elements.
+//
+// Lane p = (eta corner bit) + 2 (zeta corner bit) of an element's quad holds the two nodes
+// of its xi edge and runs the two Gauss points beside them. The derivatives at the Gauss
+// points are separable in the three directions: along one of them a difference D, along
+// the other two an interpolation to +-c (c = 1/sqrt 3), which up to a factor (1 + c)/2 is
+// own + r other with r = (1 - c)/(1 + c). xi is inside the lane, eta and zeta are shuffles
+// between the quad's lanes. The factors are the same for every derivative, so H and det F
+// do not see them and the nodal forces take them once (kHexScale). D is taken as own -
+// other on every lane: columns eta and zeta of J and G then carry the lane's signs s_eta,
+// s_zeta, which H = G J^-1 does not see either and which leave one factor s_eta s_zeta on
+// det J and on the forces. The nodal sums run the same stages transposed.
+//
+// One thread per element held the 42 coefficients of X and u and 21 sums beside a Gauss
+// point's tensors: 246 registers and eight warps per SM in FP64, and 250 warps in all on
+// 8,000 elements. A quad's lane needs 128 (FP64) or 96 registers and a quarter of the
+// serial work. Measured on B200 (1965 MHz), one thread per element against this kernel:
+// a step of 20^3 linear elastic FP64 10.8 -> 7.7 us; 128^3 neo-Hookean with fields, per
+// launch, FP64 523 -> 459 us, mixed 320 -> 306 us. FP64: the FP64 pipe is 53% busy (its
+// floor is 290 us at 128^3), gather latency takes the rest; mixed: L1 wavefronts (gathers,
+// shuffles and slot stores) 60% and gather latency. The mixed path packs the lane's two
+// Gauss points into sm_100's two-wide FP32 operations.
+// ---------------------------------------------------------------------------
+constexpr double kHexR = 0.26794919243112270647;   // (1 - c) / (1 + c) = 2 - sqrt 3
+constexpr double kHexScale = 0.31100423396407310780;  // (1 + c)^2 / 8: derivative = kHexScale x raw
+constexpr int kHexBlock = 128;
+
+template <typename T>
+struct HexPair {
+    T a, b;  // at the xi = -1 and xi = +1 nodes (or Gauss points) of the lane
+};
+__device__ __forceinline__ HexPair<float> hp_fma(float k, const HexPair<float>& x, const HexPair<float>& y) {
+    const float2 v = vfma(make_float2(k, k), make_float2(x.a, x.b), make_float2(y.a, y.b));
+    return {v.x, v.y};
+}
+__device__ __forceinline__ HexPair<double> hp_fma(double k, const HexPair<double>& x, const HexPair<double>& y) {
+    return {fma(k, x.a, y.a), fma(k, x.b, y.b)};
+}
+template <typename T>
+__device__ __forceinline__ HexPair<T> hp_xor(const HexPair<T>& x, int mask) {
+    return {__shfl_xor_sync(kFull, x.a, mask), __shfl_xor_sync(kFull, x.b, mask)};
+}
+// The xi interpolation (its own transpose).
+template <typename T>
+__device__ __forceinline__ HexPair<T> hp_interp(const HexPair<T>& x) {
+    const T r = T(kHexR);
+    return {fma(r, x.b, x.a), fma(r, x.a, x.b)};
+}
+__device__ __forceinline__ HexPair<float> hp_scale(float k, const HexPair<float>& x) {
+    const float2 v = vmul(make_float2(k, k), make_float2(x.a, x.b));
+    return {v.x, v.y};
+}
+__device__ __forceinline__ HexPair<double> hp_scale(double k, const HexPair<double>& x) { return {k * x.a, k * x.b}; }
+
+// Raw derivatives of one component at the lane's two Gauss points: d0 (xi, the same at
+// both), d1 (eta), d2 (zeta).
+template <typename T>
+__device__ __forceinline__ void hex_derivatives(const HexPair<T>& v, T& d0, HexPair<T>& d1, HexPair<T>& d2) {
+    const T r = T(kHexR);
+    const HexPair<T> q = hp_xor(v, 1);
+    const HexPair<T> D = hp_fma(T(-1), q, v), I = hp_fma(r, q, v);
+    const HexPair<T> Dz = hp_xor(D, 2), Iz = hp_xor(I, 2);
+    d1 = hp_interp(hp_fma(r, Dz, D));
+    d2 = hp_interp(hp_fma(T(-1), Iz, I));
+    d0 = fma(r, Iz.b - Iz.a, I.b - I.a);
+}
+// The transpose: z the xi terms summed over the two points, y1 and y2 the eta and zeta terms.
+template <typename T>
+__device__ __forceinline__ HexPair<T> hex_transpose(T z, const HexPair<T>& q1, const HexPair<T>& q2) {
+    const T r = T(kHexR);
+    const HexPair<T> j0{-z, z}, y1 = hp_interp(q1), y2 = hp_interp(q2);
+    const HexPair<T> w = hp_fma(T(1), hp_xor(hp_fma(-r, j0, y2), 2), hp_fma(T(1), j0, y2));
+    const HexPair<T> v = hp_fma(-r, hp_xor(y1, 2), y1);
+    return hp_fma(T(1), hp_xor(hp_fma(-r, w, v), 1), hp_fma(T(1), w, v));
+}
+
+// Q = adj(J) P^T at a Gauss point (two for float2) from J and the displacement gradient G
+// in the same raw units; sig = s_eta s_zeta. Returns whether det J and (neo-Hookean) det F
+// are positive.
+template <typename V, int MAT>
+__device__ __forceinline__ bool hex_gauss_q(const V* J, const V* G, double lam, double mu, double sig, V* Q) {
+    V A[9];
+    vadj3(J, A);
+    const V det = vfma(J[2], A[6], vfma(J[1], A[3], vmul(J[0], A[0])));
+    bool ok = all_positive(vmul(vset<V>(sig), det));
+    const V id = vrecip(det);
+    V H[9];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
-        for (int k = 0; k < 8; ++k) R[i][k] = T(0);
-    bool bad = false;
-#pragma unroll kHexGpUnroll
-    for (int g = 0; g < 8; ++g) {
-        T J[9], G[9], A[9];
+        for (int j = 0; j < 3; ++j)
+            H[i * 3 + j] = vmul(vfma(G[i * 3 + 2], A[6 + j], vfma(G[i * 3 + 1], A[3 + j], vmul(G[i * 3 + 0], A[j]))), id);
+    const V m = vset<V>(mu);
+    if (MAT == kNeoHookean) {
+        // Q = adj(J) P^T with P = tau F^-T and F = (J + G) J^-1 is adj(J + G) tau / det F
+        // (the scale of J and G cancels): no F^-1 and no P.
+        V lln, iJ;
+        ok = nh_scalars(H, lam, lln, iJ) && ok;
+        const V sm = vmul(m, iJ), sl = vmul(lln, iJ);
+        V ts[9];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                J[i * 3 + j] = hex_dxi(X[i], j, g);
-                G[i * 3 + j] = hex_dxi(U[i], j, g);
+            for (int j = i; j < 3; ++j) {
+                V t = vadd(H[i * 3 + j], H[j * 3 + i]);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) t = vfma(H[i * 3 + k], H[j * 3 + k], t);
+                t = i == j ? vfma(sm, t, sl) : vmul(sm, t);
+                ts[i * 3 + j] = ts[j * 3 + i] = t;
             }
-        adj3(J, A);
-        const T det = J[0] * A[0] + J[1] * A[3] + J[2] * A[6];
-        bad |= !(det > T(0));
-        const T id = recip(det);
-        T H[9], P[9];
+        V Jc[9], Ac[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) Jc[k] = vadd(J[k], G[k]);
+        vadj3(Jc, Ac);
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                Q[k * 3 + i] = vfma(Ac[k * 3 + 2], ts[6 + i], vfma(Ac[k * 3 + 1], ts[3 + i], vmul(Ac[k * 3 + 0], ts[i])));
+        return ok;
+    }
+    V P[9];
+    const V l = vset<V>(lam);
+    if (MAT == kLinearElastic) {
+        const V tr = vmul(l, vadd(vadd(H[0], H[4]), H[8]));
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = i; j < 3; ++j) {
+                const V e = vadd(H[i * 3 + j], H[j * 3 + i]);
+                P[i * 3 + j] = P[j * 3 + i] = i == j ? vfma(m, e, tr) : vmul(m, e);
+            }
+    } else {
+        // 2E = H + H^T + H^T H, S = lambda/2 tr(2E) I + mu 2E, P = S + H S
+        V E[9];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = i; j < 3; ++j) {
+                V e = vadd(H[i * 3 + j], H[j * 3 + i]);
+#pragma unroll
+                for (int k = 0; k < 3; ++k) e = vfma(H[k * 3 + i], H[k * 3 + j], e);
+                E[i * 3 + j] = E[j * 3 + i] = e;
+            }
+        const V tr = vmul(vset<V>(0.5 * lam), vadd(vadd(E[0], E[4]), E[8]));
+        V S[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) S[k] = k % 4 == 0 ? vfma(m, E[k], tr) : vmul(m, E[k]);
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int j = 0; j < 3; ++j)
-                H[i * 3 + j] = (G[i * 3 + 0] * A[0 * 3 + j] + G[i * 3 + 1] * A[1 * 3 + j] + G[i * 3 + 2] * A[2 * 3 + j]) * id;
-        T Q[9];
-        if (MAT == kNeoHookean) {
-            // Q = adj(J) P^T with P = tau F^-T and F = (J + G) J^-1 is adj(J + G) tau / det F
-            // (the 8x scale of J and G cancels): no F^-1 and no P.
-            T tau[9];
-            const double Jf = nh_kirchhoff<T>(T(lam), T(mu), H, tau);
-            bad |= !(Jf > 0.0);
-            T Jc[9], Ac[9];
+                P[i * 3 + j] = vfma(H[i * 3 + 2], S[6 + j], vfma(H[i * 3 + 1], S[3 + j], vfma(H[i * 3 + 0], S[j], S[i * 3 + j])));
+    }
 #pragma unroll
-            for (int k = 0; k < 9; ++k) Jc[k] = J[k] + G[k];
-            adj3(Jc, Ac);
-            const T sc = sizeof(T) == 4 ? T(__frcp_rn(static_cast<float>(Jf))) : T(1.0 / Jf);
-            T ts[9];
+    for (int k = 0; k < 3; ++k)
 #pragma unroll
-            for (int i = 0; i < 3; ++i)
-#pragma unroll
-                for (int j = i; j < 3; ++j) ts[i * 3 + j] = ts[j * 3 + i] = sc * tau[i * 3 + j];
-#pragma unroll
-            for (int k = 0; k < 3; ++k)
-#pragma unroll
-                for (int i = 0; i < 3; ++i)
-                    Q[k * 3 + i] = Ac[k * 3 + 0] * ts[0 * 3 + i] + Ac[k * 3 + 1] * ts[1 * 3 + i] + Ac[k * 3 + 2] * ts[2 * 3 + i];
-        } else {
-            stress<T>(MAT, T(lam), T(mu), H, P);
-#pragma unroll
-            for (int k = 0; k < 3; ++k)
-#pragma unroll
-                for (int i = 0; i < 3; ++i)
-                    Q[k * 3 + i] = A[k * 3 + 0] * P[i * 3 + 0] + A[k * 3 + 1] * P[i * 3 + 1] + A[k * 3 + 2] * P[i * 3 + 2];
+        for (int i = 0; i < 3; ++i)
+            Q[k * 3 + i] = vfma(A[k * 3 + 2], P[i * 3 + 2], vfma(A[k * 3 + 1], P[i * 3 + 1], vmul(A[k * 3 + 0], P[i * 3 + 0])));
+    return ok;
+}
+
+// The two nodes of corners 2p, 2p + 1 of element e from a per-node table (nodes (0,1), (3,2),
+// (4,5), (7,6)).
+__device__ __forceinline__ int2 hex_edge_pair(const int32_t* per_node, int64_t e, int p) {
+    const int2 q = reinterpret_cast<const int2*>(per_node)[4 * e + p];
+    return p & 1 ? make_int2(q.y, q.x) : q;
+}
+
+// A lane's two nodes and the element's node 0 of a nodal field, as loaded, and the two values
+// relative to node 0 (FP64 differences, then T).
+struct HexRaw {
+    double4 o, a, b;
+    template <bool DEP>
+    __device__ __forceinline__ void load(const double4* __restrict__ A, int32_t n0, int2 n) {
+        o = DEP ? ld_dep(A + n0) : ld_ro4(A + n0);
+        a = DEP ? ld_dep(A + n.x) : ld_ro4(A + n.x);
+        b = DEP ? ld_dep(A + n.y) : ld_ro4(A + n.y);
+    }
+    template <typename T>
+    __device__ __forceinline__ void rel(HexPair<T>* v) const {
+        v[0] = {T(a.x - o.x), T(b.x - o.x)};
+        v[1] = {T(a.y - o.y), T(b.y - o.y)};
+        v[2] = {T(a.z - o.z), T(b.z - o.z)};
+    }
+};
+
+// Sixteen (FP64, 128 registers) or twenty (FP32) warps per SM.
+template <typename T>
+constexpr int hex_min_blocks() { return sizeof(T) == 4 ? 5 : 4; }
+
+// Rounds of eight elements a warp runs: as many as keep three waves of 148 x 16 warps, at
+// most eight. From the second round on a warp has its connectivity at hand. Measured on
+// B200 at 128^3, neo-Hookean with fields (us per launch, 1 / 2 / 4 / 8 rounds): FP64 497 /
+// 480 / 476 / 459, mixed 344 / 321 / 311 / 306. Fewer waves leave SMs empty: 20^3 linear elastic FP64 took
+// 7.7 us a step with one round, 8.1 with two and 11.7 with four.
+inline int32_t hex_rounds(int64_t groups) { return static_cast<int32_t>(std::clamp<int64_t>(groups / (3 * 148 * 16), 1, 8)); }
+
+template <typename T, int MAT>
+__global__ void __launch_bounds__(kHexBlock, hex_min_blocks<T>()) k_hex8_force(GaussBlockDev b, const double4* __restrict__ X4,
+                                                          const double4* __restrict__ U4,
+                                                          vec4_t<T>* __restrict__ slots, int* status, int32_t rounds) {
+    constexpr int W = kHexBlock / 32;
+    const int lane = static_cast<int>(threadIdx.x & 31), p = lane & 3;
+    const int32_t E = static_cast<int32_t>(b.num_elems);
+    // the block's groups: rounds of one per warp
+    int32_t g = static_cast<int32_t>(blockIdx.x) * rounds * W + static_cast<int32_t>(threadIdx.x >> 5);
+    const int32_t last = min(g + rounds * W, (E + 7) >> 3);
+    // lanes past the last element run a copy of it (never written): the whole warp shuffles
+    const auto elem = [&](int32_t grp) { return min(8 * grp + (lane >> 2), E - 1); };
+    pdl_trigger();
+    if (g >= last) return;
+    int2 n = hex_edge_pair(b.conn, elem(g), p);
+    int32_t n0 = b.conn[8 * elem(g)];
+    const double sig = (p == 1 || p == 2) ? -1.0 : 1.0;
+    for (; g < last; g += W) {
+        const int32_t e = elem(g);
+        HexRaw X, U;
+        X.load<false>(X4, n0, n);
+        double lam, mu;
+        element_lame(b, e, lam, mu);
+        const int2 pos = hex_edge_pair(b.slot_pos, e, p);
+        pdl_wait();  // at once after the first round
+        U.load<true>(U4, n0, n);
+        // the next group's connectivity travels while this one is computed
+        if (g + W < last) {
+            n = hex_edge_pair(b.conn, elem(g + W), p);
+            n0 = b.conn[8 * elem(g + W)];
         }
-        hex_accumulate_r(R, Q, g);
-    }
-    if (bad) flag(status, AM_ENONPOS_J, e);
+        HexPair<T> x[3], u[3];
+        X.rel<T>(x);
+        U.rel<T>(u);
+        T J0[3], G0[3];
+        HexPair<T> J1[3], J2[3], G1[3], G2[3];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        R[i][0] = T(0);
-        hex_scale_coeffs(R[i]);
-        hex_butterfly_t(R[i]);
-    }
-    const T s = T(-1.0 / 512.0);
-    const int4 p0 = reinterpret_cast<const int4*>(b.slot_pos)[2 * e], p1 = reinterpret_cast<const int4*>(b.slot_pos)[2 * e + 1];
-    const int32_t pos[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+        for (int i = 0; i < 3; ++i) hex_derivatives(x[i], J0[i], J1[i], J2[i]);
 #pragma unroll
-    for (int q = 0; q < 8; ++q) slots[pos[hex_node_of_corner(q)]] = make4(s * R[0][q], s * R[1][q], s * R[2][q]);
+        for (int i = 0; i < 3; ++i) hex_derivatives(u[i], G0[i], G1[i], G2[i]);
+        T z[3];
+        HexPair<T> q1[3], q2[3];
+        bool ok;
+        if constexpr (sizeof(T) == 4) {
+            float2 J[9], G[9], Q[9];
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                J[3 * i] = make_float2(J0[i], J0[i]);
+                J[3 * i + 1] = make_float2(J1[i].a, J1[i].b);
+                J[3 * i + 2] = make_float2(J2[i].a, J2[i].b);
+                G[3 * i] = make_float2(G0[i], G0[i]);
+                G[3 * i + 1] = make_float2(G1[i].a, G1[i].b);
+                G[3 * i + 2] = make_float2(G2[i].a, G2[i].b);
+            }
+            ok = hex_gauss_q<float2, MAT>(J, G, lam, mu, sig, Q);
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                z[i] = Q[i].x + Q[i].y;
+                q1[i] = {Q[3 + i].x, Q[3 + i].y};
+                q2[i] = {Q[6 + i].x, Q[6 + i].y};
+            }
+        } else {
+            ok = true;
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                double J[9], G[9], Q[9];
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    J[3 * i] = J0[i];
+                    J[3 * i + 1] = h ? J1[i].b : J1[i].a;
+                    J[3 * i + 2] = h ? J2[i].b : J2[i].a;
+                    G[3 * i] = G0[i];
+                    G[3 * i + 1] = h ? G1[i].b : G1[i].a;
+                    G[3 * i + 2] = h ? G2[i].b : G2[i].a;
+                }
+                ok = hex_gauss_q<double, MAT>(J, G, lam, mu, sig, Q) && ok;
+#pragma unroll
+                for (int i = 0; i < 3; ++i) {
+                    if (h == 0) {
+                        z[i] = Q[i];
+                        q1[i].a = Q[3 + i];
+                        q2[i].a = Q[6 + i];
+                    } else {
+                        z[i] += Q[i];
+                        q1[i].b = Q[3 + i];
+                        q2[i].b = Q[6 + i];
+                    }
+                }
+            }
+        }
+        const bool valid = 8 * g + (lane >> 2) < E;
+        if (!ok && valid) flag(status, AM_ENONPOS_J, e);
+        const T s = T(-sig * kHexScale * kHexScale * kHexScale);
+        HexPair<T> f[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) f[i] = hp_scale(s, hex_transpose(z[i], q1[i], q2[i]));
+        if (valid) {
+            slots[pos.x] = make4(f[0].a, f[1].a, f[2].a);
+            slots[pos.y] = make4(f[0].b, f[1].b, f[2].b);
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -3251,11 +3454,13 @@ void launch_gauss_force(const GaussBlockDev& b, int mixed, const double4* X4, co
             AM_DISPATCH_MAT(b.material, (k_tet4_force<double, M><<<grid, 256, 0, s>>>(b, X4, U4, static_cast<double4*>(slots), status)));
         }
     } else {
-        const unsigned grid = grid_for(b.num_elems, 128);
+        const int64_t groups = (b.num_elems + 7) / 8;
+        const int32_t rounds = hex_rounds(groups);
+        const unsigned grid = grid_for(groups, rounds * (kHexBlock / 32));
         if (mixed) {
-            AM_DISPATCH_MAT(b.material, (launch_pdl(k_hex8_force<float, M>, grid, 128, s, b, X4, U4, static_cast<float4*>(slots), status)));
+            AM_DISPATCH_MAT(b.material, (launch_pdl(k_hex8_force<float, M>, grid, kHexBlock, s, b, X4, U4, static_cast<float4*>(slots), status, rounds)));
         } else {
-            AM_DISPATCH_MAT(b.material, (launch_pdl(k_hex8_force<double, M>, grid_for(b.num_elems, 64), 64, s, b, X4, U4, static_cast<double4*>(slots), status)));
+            AM_DISPATCH_MAT(b.material, (launch_pdl(k_hex8_force<double, M>, grid, kHexBlock, s, b, X4, U4, static_cast<double4*>(slots), status, rounds)));
         }
     }
 }

@@ -34,18 +34,26 @@ inline bool build_warp_chunks(const int32_t* conn, int64_t E, int nn, WarpChunks
     t.rank.assign(static_cast<size_t>(32 * W * C), 0xFFFFFFFFu);
     std::vector<int32_t> node(Q);
     std::vector<int> which(Q), count(Q + 1), fill(Q);
+    // rank + 1 of the chunk's nodes seen so far by a hash of the node id (linear probing;
+    // at most 256 of the 1024 places fill up)
+    std::vector<int16_t> seen(1024);
     for (int64_t c = 0; c < C; ++c) {
         const int64_t e0 = 32 * c;
         const int n = static_cast<int>(std::min<int64_t>(32, E - e0));
         std::fill(count.begin(), count.end(), 0);
+        std::fill(seen.begin(), seen.end(), int16_t{0});
         int nd = 0;
         for (int q = 0; q < Q; ++q) {
             which[q] = -1;
             if ((q & 31) >= n) continue;
             const int32_t v = conn[nn * (e0 + (q & 31)) + (q >> 5)];
-            int k = 0;
-            while (k < nd && node[k] != v) ++k;
-            if (k == nd) node[nd++] = v;
+            uint32_t h = (static_cast<uint32_t>(v) * 2654435761u) >> 22;
+            while (seen[h] != 0 && node[seen[h] - 1] != v) h = (h + 1) & 1023u;
+            if (seen[h] == 0) {
+                node[nd++] = v;
+                seen[h] = static_cast<int16_t>(nd);
+            }
+            const int k = seen[h] - 1;
             which[q] = k;
             ++count[k + 1];
         }

@@ -833,8 +833,11 @@ struct am_ctx {
             // (StepScheduler at update_interval, src/Application.cpp:301-308): the element
             // kernels take the stored H as the reference gradient first.
             const int rebase = (lagr == 2 && lagr_steps > 0 && lagr_steps % lagr_interval == 0 && !lagr_rebased) ? 1 : 0;
+            // The H of this evaluation is read again as a reference gradient only by the next
+            // step (updated), or by the step after a reference update (semi): kept only then.
+            const int keep = (lagr == 1 || (lagr_steps + 1) % lagr_interval == 0) ? 1 : 0;
             for (auto& b : blocks) {
-                am::launch_gauss_force_lagr(b.gauss(), lagr, rebase, xc, lagr_inc, s, status, stream);
+                am::launch_gauss_force_lagr(b.gauss(), lagr, rebase, keep, xc, lagr_inc, s, status, stream);
                 ++launches;
             }
             if (rebase) lagr_rebased = true;
@@ -1745,10 +1748,11 @@ int am_add_block(am_ctx* ctx, const am_block_desc* d, int32_t* block_id) {
                     am::launch_tet4_geometry(b.conn, E, ctx->X4, b.geo32, b.geo64, ctx->stream);
                     ck(cudaGetLastError(), "tet geometry");
                 }
-                // Warp chunks for the one-thread-per-tet kernel (Hex8 measured no gain: its
+                // Warp chunks for the one-thread-per-tet kernels (Hex8 measured no gain: its
                 // issue-bound element kernel paid for the warp sums what its node kernel saved).
                 WarpChunks wc;
-                if (ctx->warp_chunks && E > 0 && d->kind == AM_TET4_GAUSS && b.geo64 && build_warp_chunks(conn, E, nn, wc))
+                if (ctx->warp_chunks && E > 0 && d->kind == AM_TET4_GAUSS && (b.geo64 || ctx->lagr != 0) &&
+                    build_warp_chunks(conn, E, nn, wc))
                     upload_warp_chunks(b, wc, E);
             }
             if (ctx->num_slots + b.num_entries >= (int64_t(1) << 31)) fail(AM_ERANGE, "slot count beyond int32 indexing");

@@ -60,6 +60,9 @@ __device__ __forceinline__ double4 ld_ro4(const double4* p) {
     return r;
 }
 
+// Sends a line that is read later (past other loads' latency) to L2.
+__device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
+
 __device__ __forceinline__ void flag(int* status, int code, int64_t idx) {
     if (status == nullptr) return;
     if (atomicCAS(status + kStatusCode, 0, code) == 0) status[kStatusIndex] = static_cast<int>(idx);
@@ -1160,12 +1163,12 @@ __global__ void __launch_bounds__(kHexBlock, hex_min_blocks<T>()) k_hex8_force(G
 // The element H arrays are component-major (component k of element e at k E + e), so that a
 // warp's nine loads and stores are coalesced. They are written by the element kernel of the
 // previous step: read after the wait for the predecessor, with coherent loads.
-__device__ __forceinline__ void lagr_href(const GaussBlockDev& b, int64_t e, int32_t lagr, int rebase, double* hr) {
+__device__ __forceinline__ void lagr_href(const GaussBlockDev& b, int64_t e, int32_t lagr, int rebase, bool own, double* hr) {
     const int64_t E = b.num_elems;
     const double* src = (lagr == 1 || rebase) ? b.hstate : b.href;
 #pragma unroll
     for (int k = 0; k < 9; ++k) hr[k] = __ldcg(src + k * E + e);
-    if (lagr == 2 && rebase) {
+    if (lagr == 2 && rebase && own) {
 #pragma unroll
         for (int k = 0; k < 9; ++k) b.href[k * E + e] = hr[k];
     }
@@ -1198,17 +1201,40 @@ __device__ __forceinline__ void lagr_pull(const double* hr, const double* P, dou
             Pm[i * 3 + m] = (P[i * 3 + 0] * Fr[m * 3 + 0] + P[i * 3 + 1] * Fr[m * 3 + 1] + P[i * 3 + 2] * Fr[m * 3 + 2]) * idet;
 }
 
-template <int MAT>
-__global__ void __launch_bounds__(128) k_tet4_force_lagr(GaussBlockDev b, int32_t lagr, int rebase,
+// One thread per tet. CHUNKS: the warp's 32 tets sum their shared nodes as in
+// k_tet4_force_geo. keep: this evaluation's H may become a reference gradient (every step
+// under the updated formulation, the last step before a reference update under the semi
+// one); otherwise it is not written. A tet reads its H_ref before its gathers, so that the
+// one wait covers both. Latency of those loads binds (FP64 pipe 36%), hence 20 warps per SM
+// for a few spilled registers. On a 45 x 45 x 61 box (741,150 tets, B200, 1965 MHz, semi with
+// an update every 10 steps), us per step: four slots per tet and H written every step 79.8;
+// chunks and keep 60.4; H_ref first 55.3; 20 warps 51.4 (24 warps, more spills: 52.3).
+template <int MAT, bool CHUNKS>
+__global__ void __launch_bounds__(128, 5) k_tet4_force_lagr(GaussBlockDev b, int32_t lagr, int rebase, int keep,
                                                           const double4* __restrict__ XC,
                                                           const double4* __restrict__ INC,
                                                           double4* __restrict__ slots, int* status) {
     pdl_trigger();
-    const int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (e >= b.num_elems) return;
+    const int64_t E = b.num_elems;
+    const int64_t et = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    // chunked: lanes past the last tet run a copy of it (never summed, nothing kept) to
+    // reach the warp sum
+    if (!CHUNKS && et >= E) return;
+    const bool own = et < E;
+    const int64_t e = own ? et : E - 1;
     const int4 c = reinterpret_cast<const int4*>(b.conn)[e];
-    const int32_t pos[4] = {b.slot_pos[4 * e], b.slot_pos[4 * e + 1], b.slot_pos[4 * e + 2], b.slot_pos[4 * e + 3]};
+    int32_t pos[4] = {0, 0, 0, 0};
+    if (CHUNKS) {
+        prefetch_l2(b.chunk_code + e);
+        prefetch_l2(b.chunk_rank + e);
+        prefetch_l2(b.chunk_pos + 4 * e);
+    } else {
+#pragma unroll
+        for (int a = 0; a < 4; ++a) pos[a] = b.slot_pos[4 * e + a];
+    }
     pdl_wait();
+    double dH[9], hr[9], H[9];
+    lagr_href(b, e, lagr, rebase, own, hr);
     const double4 x0 = ld_dep(XC + c.x), x1 = ld_dep(XC + c.y), x2 = ld_dep(XC + c.z), x3 = ld_dep(XC + c.w);
     const double4 u0 = ld_dep(INC + c.x), u1 = ld_dep(INC + c.y), u2 = ld_dep(INC + c.z), u3 = ld_dep(INC + c.w);
     const double J[9] = {x1.x - x0.x, x2.x - x0.x, x3.x - x0.x, x1.y - x0.y, x2.y - x0.y,
@@ -1216,23 +1242,21 @@ __global__ void __launch_bounds__(128) k_tet4_force_lagr(GaussBlockDev b, int32_
     const double D[9] = {u1.x - u0.x, u2.x - u0.x, u3.x - u0.x, u1.y - u0.y, u2.y - u0.y,
                          u3.y - u0.y, u1.z - u0.z, u2.z - u0.z, u3.z - u0.z};
     const double det = det3(J);
-    if (!(det > 0.0)) flag(status, AM_ENONPOS_J, e);
+    if (own && !(det > 0.0)) flag(status, AM_ENONPOS_J, e);
     double Ji[9];
     cof_inv3(J, Ji, det);
     const double w = det / 6.0;
-    double dH[9], hr[9], H[9];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = 0; j < 3; ++j) dH[i * 3 + j] = D[i * 3 + 0] * Ji[0 * 3 + j] + D[i * 3 + 1] * Ji[1 * 3 + j] + D[i * 3 + 2] * Ji[2 * 3 + j];
-    lagr_href(b, e, lagr, rebase, hr);
     lagr_compose(dH, hr, H);
-    lagr_store_h(b, e, H);
+    if (keep && own) lagr_store_h(b, e, H);
     double lam, mu;
     element_lame(b, e, lam, mu);
     double P[9], Pm[9];
     const double Jf = stress<double>(MAT, lam, mu, H, P);
-    if (MAT == kNeoHookean && !(Jf > 0.0)) flag(status, AM_ENONPOS_J, e);
+    if (own && MAT == kNeoHookean && !(Jf > 0.0)) flag(status, AM_ENONPOS_J, e);
     lagr_pull(hr, P, Pm);
     double f[12];
 #pragma unroll
@@ -1245,14 +1269,31 @@ __global__ void __launch_bounds__(128) k_tet4_force_lagr(GaussBlockDev b, int32_
             f[(k + 1) * 3 + i] = -q;
             f[i] += q;
         }
-    slots[pos[0]] = make4(f[0], f[1], f[2]);
-    slots[pos[1]] = make4(f[3], f[4], f[5]);
-    slots[pos[2]] = make4(f[6], f[7], f[8]);
-    slots[pos[3]] = make4(f[9], f[10], f[11]);
+    if constexpr (!CHUNKS) {
+#pragma unroll
+        for (int a = 0; a < 4; ++a) slots[pos[a]] = make4(f[3 * a], f[3 * a + 1], f[3 * a + 2]);
+    } else {
+        __shared__ double ent[128 / 32][3][128];
+        double(&st)[3][128] = ent[threadIdx.x >> 5];
+        const int lane = static_cast<int>(threadIdx.x & 31);
+#pragma unroll
+        for (int a = 0; a < 4; ++a)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) st[i][32 * a + lane] = f[3 * a + i];
+        __syncwarp();
+        const int64_t ch = et >> 5;
+        if (32 * ch >= E) return;  // the whole warp
+        const ChunkLane<4> L = chunk_lane<4>(b, ch, lane, true);
+        chunk_reduce<double, 4>(L, lane, [&](int q, double(&v)[3]) {
+            v[0] = st[0][q];
+            v[1] = st[1][q];
+            v[2] = st[2][q];
+        }, slots);
+    }
 }
 
 template <int MAT>
-__global__ void __launch_bounds__(64) k_hex8_force_lagr(GaussBlockDev b, int32_t lagr, int rebase,
+__global__ void __launch_bounds__(64) k_hex8_force_lagr(GaussBlockDev b, int32_t lagr, int rebase, int keep,
                                                          const double4* __restrict__ XC,
                                                          const double4* __restrict__ INC,
                                                          double4* __restrict__ slots, int* status) {
@@ -1275,7 +1316,7 @@ __global__ void __launch_bounds__(64) k_hex8_force_lagr(GaussBlockDev b, int32_t
     double lam, mu;
     element_lame(b, e, lam, mu);
     double hr[9];
-    lagr_href(b, e, lagr, rebase, hr);
+    lagr_href(b, e, lagr, rebase, true, hr);
     double R[3][8];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
@@ -1303,7 +1344,7 @@ __global__ void __launch_bounds__(64) k_hex8_force_lagr(GaussBlockDev b, int32_t
                 dH[i * 3 + j] = (G[i * 3 + 0] * A[0 * 3 + j] + G[i * 3 + 1] * A[1 * 3 + j] + G[i * 3 + 2] * A[2 * 3 + j]) * id;
         lagr_compose(dH, hr, H);
         // The reference's last Gauss point (its node 7 sign pattern) is corner 6 here.
-        if (g == 6) lagr_store_h(b, e, H);
+        if (g == 6 && keep) lagr_store_h(b, e, H);
         const double Jf = stress<double>(MAT, lam, mu, H, P);
         if (MAT == kNeoHookean) bad |= !(Jf > 0.0);
         lagr_pull(hr, P, Pm);
@@ -3873,14 +3914,16 @@ void launch_pm_scale(int64_t n, double4* V4, double scale, cudaStream_t s) {
     if (n > 0) k_pm_scale<<<grid_for(n, 256), 256, 0, s>>>(n, V4, scale);
 }
 
-void launch_gauss_force_lagr(const GaussBlockDev& b, int32_t lagr, int rebase, const double4* XC, const double4* INC,
-                             void* slots, int* status, cudaStream_t s) {
+void launch_gauss_force_lagr(const GaussBlockDev& b, int32_t lagr, int rebase, int keep, const double4* XC,
+                             const double4* INC, void* slots, int* status, cudaStream_t s) {
     if (b.num_elems == 0) return;
     double4* sl = static_cast<double4*>(slots);
     if (b.kind == AM_HEX8_GAUSS) {
-        AM_DISPATCH_MAT(b.material, (launch_pdl(k_hex8_force_lagr<M>, grid_for(b.num_elems, 64), 64, s, b, lagr, rebase, XC, INC, sl, status)));
+        AM_DISPATCH_MAT(b.material, (launch_pdl(k_hex8_force_lagr<M>, grid_for(b.num_elems, 64), 64, s, b, lagr, rebase, keep, XC, INC, sl, status)));
+    } else if (b.chunk_ptr != nullptr) {
+        AM_DISPATCH_MAT(b.material, (launch_pdl(k_tet4_force_lagr<M, true>, grid_for(b.num_elems, 128), 128, s, b, lagr, rebase, keep, XC, INC, sl, status)));
     } else {
-        AM_DISPATCH_MAT(b.material, (launch_pdl(k_tet4_force_lagr<M>, grid_for(b.num_elems, 128), 128, s, b, lagr, rebase, XC, INC, sl, status)));
+        AM_DISPATCH_MAT(b.material, (launch_pdl(k_tet4_force_lagr<M, false>, grid_for(b.num_elems, 128), 128, s, b, lagr, rebase, keep, XC, INC, sl, status)));
     }
 }
 

@@ -204,7 +204,7 @@ void launch_iface_gather(const NodeDev& nd, int mixed, const void* slots, int64_
 // Updated / semi-Lagrangian element forces (FP64): coordinates xc, displacement inc, the
 // element's reference gradient (rebase: the semi formulation's reference update takes the
 // last stored H first).
-void launch_gauss_force_lagr(const GaussBlockDev& b, int32_t lagr, int rebase, const double4* XC, const double4* INC,
+void launch_gauss_force_lagr(const GaussBlockDev& b, int32_t lagr, int rebase, int keep, const double4* XC, const double4* INC,
                              void* slots, int* status, cudaStream_t s);
 // a = (f + g m) / m with no boundary condition (pre-loop acceleration).
 void launch_init_accel(const NodeDev& nd, int mixed, const void* slots, double4* A4, int* status, cudaStream_t s);

@@ -355,7 +355,7 @@ int am_solve_power_method(am_ctx* ctx, am_precision prec, double scale_factor, i
  * starts undeformed and is reset by every am_set_state (whose displacement, null meaning
  * zero, should be zero); FP64 only; Gauss blocks only; not with am_internal_force, the VJP, the adjoint,
  * the power method, the two-pass coupling or a decomposed mesh (AM_ESTATE). Call after
- * am_create and before am_add_block (Tet4 blocks then keep per-element slots). */
+ * am_create and before am_add_block (Tet4 blocks then run one thread per tet). */
 int am_set_formulation(am_ctx* ctx, int32_t formulation, int32_t update_interval);
 
 /* ---- two-pass reproducing-kernel coupling (the solver's generalized-field path with the

@@ -103,14 +103,18 @@ void nccl_check(ncclResult_t r, const char* what) {
 // offset (partner minus item, or their anchors': on a locality-numbered mesh consecutive
 // items see the same offsets, so a row's eight partners are consecutive) when that pads by
 // at most 35% over the octet's entries; otherwise each item's entries fill rows from the
-// first. src holds, per (row, item) at 8 row + item, the entry or -1 (padding).
+// first. src holds, per (row, item) at 8 row + item, the entry or -1 (padding). index_ptr and
+// index give the rows' partners as RowIndexDev reads them (without anchors): one key per row
+// where an octet's rows are aligned, else one index per record.
 struct OctetRows {
     std::vector<int32_t> ptr;
     std::vector<int32_t> src;
+    std::vector<int32_t> index_ptr, index;
 };
 
 OctetRows octet_rows(int64_t count, const std::vector<int32_t>& ptr, const std::vector<int32_t>& partner,
-                     const int32_t* item_anchor = nullptr, const int32_t* partner_anchor = nullptr, int items = 8) {
+                     const int32_t* item_anchor = nullptr, const int32_t* partner_anchor = nullptr, int items = 8,
+                     bool with_index = false) {
     if (items == 1) {
         // a warp per item: its rows are its entries
         OctetRows o;
@@ -129,7 +133,7 @@ OctetRows octet_rows(int64_t count, const std::vector<int32_t>& ptr, const std::
     const int64_t O = (count + 7) / 8;
     o.ptr.reserve(O + 1);
     o.ptr.push_back(0);
-    std::vector<int32_t> rowsrc;
+    std::vector<int32_t> rowsrc, rowkey;
     for (int64_t q = 0; q < O; ++q) {
         int32_t at[8], end[8];
         int64_t total = 0, longest = 0;
@@ -142,6 +146,7 @@ OctetRows octet_rows(int64_t count, const std::vector<int32_t>& ptr, const std::
         }
         // aligned rows: merge the offset lists, a row per offset (times its largest multiplicity)
         rowsrc.clear();
+        rowkey.clear();
         int32_t p[8];
         std::copy(at, at + 8, p);
         while (true) {
@@ -155,12 +160,16 @@ OctetRows octet_rows(int64_t count, const std::vector<int32_t>& ptr, const std::
                 while (p[j] + run[j] < end[j] && key(8 * q + j, p[j] + run[j]) == off) ++run[j];
                 mult = std::max(mult, run[j]);
             }
-            for (int32_t t = 0; t < mult; ++t)
+            for (int32_t t = 0; t < mult; ++t) {
+                rowkey.push_back(static_cast<int32_t>(off));
                 for (int j = 0; j < 8; ++j) rowsrc.push_back(t < run[j] ? p[j] + t : -1);
+            }
             for (int j = 0; j < 8; ++j) p[j] += run[j];
         }
         const int64_t aligned = static_cast<int64_t>(rowsrc.size()) / 8;
-        if (8 * aligned * 100 <= 135 * total) {
+        const bool keep = 8 * aligned * 100 <= 135 * total;
+        const size_t first = o.src.size();
+        if (keep) {
             o.src.insert(o.src.end(), rowsrc.begin(), rowsrc.end());
             o.ptr.push_back(o.ptr.back() + static_cast<int32_t>(aligned));
         } else {
@@ -169,6 +178,14 @@ OctetRows octet_rows(int64_t count, const std::vector<int32_t>& ptr, const std::
             o.ptr.push_back(o.ptr.back() + static_cast<int32_t>(longest));
         }
         if (static_cast<int64_t>(o.src.size()) >= (int64_t(1) << 31)) fail(AM_ERANGE, "octet rows beyond int32 indexing");
+        if (!with_index) continue;
+        const int32_t at_index = static_cast<int32_t>(o.index.size());
+        o.index_ptr.push_back(keep ? ~at_index : at_index);
+        if (keep) {
+            o.index.insert(o.index.end(), rowkey.begin(), rowkey.end());
+        } else {
+            for (size_t r = first; r < o.src.size(); ++r) o.index.push_back(o.src[r] < 0 ? 0 : partner[o.src[r]]);
+        }
     }
     return o;
 }
@@ -180,6 +197,13 @@ float bits32(int32_t v) {
 }
 double bits64(int32_t v) {
     const int64_t w = v;
+    double d;
+    std::memcpy(&d, &w, sizeof d);
+    return d;
+}
+// The value of a padding record (see RowIndexDev).
+double pad64() {
+    const int64_t w = static_cast<int64_t>(am::kPadHi) << 32;
     double d;
     std::memcpy(&d, &w, sizeof d);
     return d;
@@ -749,13 +773,15 @@ struct am_ctx {
     int32_t* rkt_src = nullptr;
     double* rkt_val = nullptr;
     // The same rows and columns in warp octets (APERI_B200_RK_OCTETS=0 keeps the CSR kernels):
-    // octet row offsets and (value, index) records.
+    // octet row offsets, weights and indices (RowIndexDev).
     bool rk_octets = true;
     int64_t rko_count = 0, rkto_count = 0;
     int32_t* rko_ptr = nullptr;
     int32_t* rkto_ptr = nullptr;
-    double2* rko_rec = nullptr;
-    double2* rkto_rec = nullptr;
+    double* rko_w = nullptr;
+    double* rkto_w = nullptr;
+    int32_t *rko_iptr = nullptr, *rko_idx = nullptr;
+    int32_t *rkto_iptr = nullptr, *rkto_idx = nullptr;
     double4* rk_u = nullptr;          // physical displacement Psi U
     double4* rk_f_local = nullptr;
     double4* rk_l = nullptr;  // the cotangent at the points (VJP with the two-pass coupling)    // element forces at the nodes
@@ -812,15 +838,15 @@ struct am_ctx {
     // to the generalized force Psi^T f, which the node kernels then read (f_given).
     // The two-pass functions: Psi in (nodes) -> out (points); Psi^T in (points) -> out (nodes, N x 3).
     void rk_rows(const double4* in, double4* out) {
-        if (rko_rec)
-            am::launch_rk_octets(points(), rko_count, rko_ptr, rko_rec, in, rk_ptr, N, out, nullptr, stream);
+        if (rko_w)
+            am::launch_rk_octets(points(), rko_count, rko_ptr, rko_w, {rko_iptr, rko_idx}, in, rk_ptr, N, out, nullptr, stream);
         else
             am::launch_rk_rows4(points(), N, rk_ptr, rk_nbr, rk_val, in, out, stream);
         ++launches;
     }
     void rk_cols(const double4* in, double* out) {
-        if (rkto_rec)
-            am::launch_rk_octets(N, rkto_count, rkto_ptr, rkto_rec, in, nullptr, N, nullptr, out, stream);
+        if (rkto_w)
+            am::launch_rk_octets(N, rkto_count, rkto_ptr, rkto_w, {rkto_iptr, rkto_idx}, in, nullptr, N, nullptr, out, stream);
         else
             am::launch_rk_cols3(N, rkt_ptr, rkt_src, rkt_val, in, out, stream);
         ++launches;
@@ -1357,8 +1383,12 @@ struct am_ctx {
         dfree(rkt_val);
         dfree(rko_ptr);
         dfree(rkto_ptr);
-        dfree(rko_rec);
-        dfree(rkto_rec);
+        dfree(rko_w);
+        dfree(rkto_w);
+        dfree(rko_iptr);
+        dfree(rko_idx);
+        dfree(rkto_iptr);
+        dfree(rkto_idx);
         dfree(rk_u);
         dfree(rk_f_local);
         dfree(rk_l);
@@ -2647,16 +2677,16 @@ int am_set_rk_functions(am_ctx* ctx, const int64_t* nbr_ptr, const int32_t* nbr,
         if (ctx->rk_octets) {
             // rows sorted by node and columns (ascending point already) in warp octets
             auto octets = [&](int64_t count, const std::vector<int32_t>& ptr, const std::vector<int32_t>& part,
-                              const std::vector<double>& w, int32_t*& optr, double2*& rec, int64_t& n_oct) {
-                const OctetRows o = octet_rows(count, ptr, part);
-                std::vector<double2> h(o.src.size());
-                for (size_t q = 0; q < h.size(); ++q) {
-                    const int32_t e = o.src[q];
-                    h[q] = e < 0 ? make_double2(0.0, bits64(-1)) : make_double2(w[e], bits64(part[e]));
-                }
+                              const std::vector<double>& w, int32_t*& optr, double*& rec, int32_t*& iptr,
+                              int32_t*& idx, int64_t& n_oct) {
+                const OctetRows o = octet_rows(count, ptr, part, nullptr, nullptr, 8, true);
+                std::vector<double> h(o.src.size());
+                for (size_t q = 0; q < h.size(); ++q) h[q] = o.src[q] < 0 ? pad64() : w[o.src[q]];
+                up(iptr, o.index_ptr.data(), static_cast<int64_t>(o.index_ptr.size()), "function octet index offsets");
+                up(idx, o.index.data(), static_cast<int64_t>(o.index.size()), "function octet indices");
                 n_oct = static_cast<int64_t>(o.ptr.size()) - 1;
                 up(optr, o.ptr.data(), static_cast<int64_t>(o.ptr.size()), "function octet rows");
-                up(rec, h.data(), static_cast<int64_t>(h.size()), "function octet records");
+                up(rec, h.data(), static_cast<int64_t>(h.size()), "function octet weights");
             };
             std::vector<int32_t> rptr(NP + 1), rpart(static_cast<size_t>(K));
             std::vector<double> rval(static_cast<size_t>(K));
@@ -2673,8 +2703,10 @@ int am_set_rk_functions(am_ctx* ctx, const int64_t* nbr_ptr, const int32_t* nbr,
             }
             rptr[NP] = static_cast<int32_t>(K);
             std::vector<int32_t> cptr(tptr.begin(), tptr.end());
-            octets(NP, rptr, rpart, rval, ctx->rko_ptr, ctx->rko_rec, ctx->rko_count);
-            octets(N, cptr, tsrc, tval, ctx->rkto_ptr, ctx->rkto_rec, ctx->rkto_count);
+            octets(NP, rptr, rpart, rval, ctx->rko_ptr, ctx->rko_w, ctx->rko_iptr, ctx->rko_idx,
+                    ctx->rko_count);
+            octets(N, cptr, tsrc, tval, ctx->rkto_ptr, ctx->rkto_w, ctx->rkto_iptr, ctx->rkto_idx,
+                    ctx->rkto_count);
         }
         up(ctx->rk_ptr, nbr_ptr, NP + 1, "function offsets");
         up(ctx->rk_nbr, nbr, K, "function neighbours");

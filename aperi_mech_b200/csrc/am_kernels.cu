@@ -1503,9 +1503,34 @@ __device__ __forceinline__ void warp_sum2(double& x, double& y) {
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ int32_t rec_index(const float4& r) { return __float_as_int(r.w); }
 __device__ __forceinline__ int32_t rec_index(const double4& r) { return static_cast<int32_t>(__double_as_longlong(r.w)); }
-// Records are written once at set-up: the read-only path.
-__device__ __forceinline__ float4 ld_rec(const float4* p) { return __ldg(p); }
-__device__ __forceinline__ double4 ld_rec(const double4* p) { return ld_ro4(p); }
+// Records are written once at set-up and read once per evaluation: the read-only path, past
+// the L1 that the u and M gathers reuse, and first to leave L2. On B200, 70,785 RKPM cells in
+// FP32: 51.7 -> 48.0 us a step past L1 (the L2 policy changes nothing there); 384,000 F-bar
+// subcells in FP64: 220 -> 206 us a step with the L2 policy (218 with it on one side only).
+// Apart, the FP64 gradient and index are 28 bytes in three loads instead of 32 in one, and
+// slower: 237 us at best.
+__device__ __forceinline__ uint64_t stream_policy() {
+    uint64_t q;
+    asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(q));
+    return q;
+}
+__device__ __forceinline__ float4 ld_stream(const float4* p, uint64_t q) {
+    float4 r;
+    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+        : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(p), "l"(q));
+    return r;
+}
+__device__ __forceinline__ double4 ld_stream(const double4* p, uint64_t q) {
+    double4 r;
+    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v4.f64 {%0, %1, %2, %3}, [%4], %5;"
+        : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p), "l"(q));
+    return r;
+}
+__device__ __forceinline__ double ld_stream(const double* p, uint64_t q) {
+    double r;
+    asm("ld.global.nc.L1::no_allocate.L2::cache_hint.f64 %0, [%1], %2;" : "=d"(r) : "l"(p), "l"(q));
+    return r;
+}
 template <typename T>
 __device__ __forceinline__ vec4_t<T> pad_rec() {
     vec4_t<T> z;
@@ -1570,9 +1595,10 @@ __global__ void __launch_bounds__(256) k_cell_stress(CellBlockDev b, const doubl
     const vec4_t<T>* rec = cell_recs<T>(b) + G * static_cast<int64_t>(r0) + j;
     const int32_t ref = valid ? b.c_ref[c] : -1;
     const bool diff = sizeof(T) == 4;
+    const uint64_t policy = stream_policy();
     vec4_t<T> rr[UNR];
 #pragma unroll
-    for (int u = 0; u < UNR; ++u) rr[u] = k + L * u < rows ? ld_rec(rec + G * (k + L * u)) : pad_rec<T>();
+    for (int u = 0; u < UNR; ++u) rr[u] = k + L * u < rows ? ld_stream(rec + G * (k + L * u), policy) : pad_rec<T>();
     pdl_wait();
     const double4 ur = ref >= 0 ? ld_dep(U4 + ref) : make_double4(0.0, 0.0, 0.0, 0.0);
     T H[9];
@@ -1590,7 +1616,7 @@ __global__ void __launch_bounds__(256) k_cell_stress(CellBlockDev b, const doubl
 #pragma unroll
         for (int u = 0; u < UNR; ++u) {
             const int32_t rn = r + L * (UNR + u);
-            nx[u] = rn < rows ? ld_rec(rec + G * rn) : pad_rec<T>();
+            nx[u] = rn < rows ? ld_stream(rec + G * rn, policy) : pad_rec<T>();
         }
 #pragma unroll
         for (int u = 0; u < UNR; ++u) {
@@ -1721,9 +1747,10 @@ __global__ void __launch_bounds__(256) k_cell_gather(CellBlockDev b, const T* __
     const int32_t r0 = live ? b.n_ptr[o] : 0, rows = live ? b.n_ptr[o + 1] - r0 : 0;
     const int32_t pos = valid && k == 0 ? b.slot_pos[i] : 0;
     const vec4_t<T>* rec = node_recs<T>(b) + G * static_cast<int64_t>(r0) + j;
+    const uint64_t policy = stream_policy();
     vec4_t<T> rr[UNR];
 #pragma unroll
-    for (int u = 0; u < UNR; ++u) rr[u] = k + L * u < rows ? ld_rec(rec + G * (k + L * u)) : pad_rec<T>();
+    for (int u = 0; u < UNR; ++u) rr[u] = k + L * u < rows ? ld_stream(rec + G * (k + L * u), policy) : pad_rec<T>();
     pdl_wait();
     double f[3] = {0.0, 0.0, 0.0};
 #pragma unroll 1
@@ -1743,7 +1770,7 @@ __global__ void __launch_bounds__(256) k_cell_gather(CellBlockDev b, const T* __
 #pragma unroll
         for (int u = 0; u < UNR; ++u) {
             const int32_t rn = r + L * (UNR + u);
-            nx[u] = rn < rows ? ld_rec(rec + G * rn) : pad_rec<T>();
+            nx[u] = rn < rows ? ld_stream(rec + G * rn, policy) : pad_rec<T>();
         }
 #pragma unroll
         for (int u = 0; u < UNR; ++u) {
@@ -3202,13 +3229,17 @@ __global__ void __launch_bounds__(128) k_rk_cols3(int64_t n, const int64_t* __re
 
 // The coupling in warp octets (the row layout of the cell-stress form): item i (a point for
 // the rows of Psi, a node for its columns) sums w * in[idx] over its rows, lane 8k + j taking
-// item j of the octet and rows k, k + 4, ...; records are (w, idx) pairs in one 16-byte load,
-// idx -1 for padding. Rows are aligned by offset where that pads little, so a quarter-warp's
-// eight gathers read consecutive nodes or points. Rows of Psi without neighbours copy the
-// node's coefficient (out4 set, row_ptr the original offsets); columns write out3.
+// item j of the octet and rows k, k + 4, ...; a row is eight FP64 weights and, where the
+// octet's rows are aligned by offset (a quarter-warp's eight gathers then read consecutive
+// nodes or points), one index key: 8.5 bytes per record instead of 16 with the index beside
+// the weight. Rows of Psi without neighbours copy the node's coefficient (out4 set, row_ptr
+// the original offsets); columns write out3. On 70,785 nodes (32 x 32 x 64 box, B200) the two
+// coupling launches of a step read 39 -> 24 MB each and took 17.5 -> 15.2 us; latency of the
+// gathers binds now.
 template <int UNR>
 __global__ void __launch_bounds__(256) k_rk_octets(int64_t count, int64_t num_octets, const int32_t* __restrict__ optr,
-                                                   const double2* __restrict__ rec, const double4* __restrict__ in,
+                                                   const double* __restrict__ w, RowIndexDev index,
+                                                   const double4* __restrict__ in,
                                                    const int64_t* __restrict__ row_ptr, int64_t num_nodes,
                                                    double4* __restrict__ out4, double* __restrict__ out3) {
     const int64_t o = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -3217,11 +3248,23 @@ __global__ void __launch_bounds__(256) k_rk_octets(int64_t count, int64_t num_oc
     const bool valid = i < count;
     const bool live = o < num_octets;
     const int32_t r0 = live ? optr[o] : 0, rows = live ? optr[o + 1] - r0 : 0;
-    const double2* rp = rec + 8 * static_cast<int64_t>(r0) + j;
+    const int32_t ip = live ? index.ptr[o] : 0;
+    const bool aligned = ip < 0;
+    const int32_t* idx = index.idx + (aligned ? ~ip : ip + j);
+    const int32_t step = aligned ? 1 : 8, add = aligned ? static_cast<int32_t>(i) : 0;
+    const double* wp = w + 8 * static_cast<int64_t>(r0) + j;
+    const uint64_t policy = stream_policy();
+    // a row's weight and partner (-1: padding)
+    const auto row = [&](int32_t r) {
+        const double v = ld_stream(wp + 8 * r, policy);
+        const int32_t n = __ldg(idx + step * r) + add;
+        const bool pad = __double2hiint(v) == kPadHi;
+        return make_double2(pad ? 0.0 : v, __longlong_as_double(pad ? -1LL : static_cast<long long>(n)));
+    };
     const double2 pad = make_double2(0.0, __longlong_as_double(-1LL));
     double2 rr[UNR];
 #pragma unroll
-    for (int u = 0; u < UNR; ++u) rr[u] = k + 4 * u < rows ? __ldg(rp + 8 * (k + 4 * u)) : pad;
+    for (int u = 0; u < UNR; ++u) rr[u] = k + 4 * u < rows ? row(k + 4 * u) : pad;
     double x = 0.0, y = 0.0, z = 0.0;
 #pragma unroll 1
     for (int32_t r = k; r < rows; r += 4 * UNR) {
@@ -3235,7 +3278,7 @@ __global__ void __launch_bounds__(256) k_rk_octets(int64_t count, int64_t num_oc
 #pragma unroll
         for (int u = 0; u < UNR; ++u) {
             const int32_t rn = r + 4 * (UNR + u);
-            nx[u] = rn < rows ? __ldg(rp + 8 * rn) : pad;
+            nx[u] = rn < rows ? row(rn) : pad;
         }
 #pragma unroll
         for (int u = 0; u < UNR; ++u) {
@@ -3936,10 +3979,12 @@ void launch_rk_cols3(int64_t n, const int64_t* tptr, const int32_t* tsrc, const 
     if (n > 0) k_rk_cols3<<<grid_for(n * kRkLanes, 128), 128, 0, s>>>(n, tptr, tsrc, tval, f_local, f);
 }
 
-void launch_rk_octets(int64_t count, int64_t num_octets, const int32_t* optr, const double2* rec, const double4* in,
-                      const int64_t* row_ptr, int64_t num_nodes, double4* out4, double* out3, cudaStream_t s) {
-    if (count > 0) k_rk_octets<4><<<grid_for(num_octets * 32, 256), 256, 0, s>>>(count, num_octets, optr, rec, in, row_ptr,
-                                                                                num_nodes, out4, out3);
+void launch_rk_octets(int64_t count, int64_t num_octets, const int32_t* optr, const double* w, const RowIndexDev& index,
+                      const double4* in, const int64_t* row_ptr, int64_t num_nodes, double4* out4, double* out3,
+                      cudaStream_t s) {
+    if (count > 0)
+        k_rk_octets<4><<<grid_for(num_octets * 32, 256), 256, 0, s>>>(count, num_octets, optr, w, index, in, row_ptr,
+                                                                      num_nodes, out4, out3);
 }
 
 void launch_pack4(const double* aos3, double4* out, int64_t n, cudaStream_t s) {

@@ -81,6 +81,16 @@ struct GaussBlockDev {
     double* href;
 };
 
+// Partner indices of octet rows, apart from the rows' values. ptr[o] >= 0: one index per
+// record of octet o from idx[ptr[o]] on (row r of item j at 8 r + j); ptr[o] < 0: the octet's
+// rows are aligned, row r has one key idx[~ptr[o] + r] and item i's partner is key + i.
+// Padding is marked in the record's value (kPadHi).
+struct RowIndexDev {
+    const int32_t* ptr;
+    const int32_t* idx;
+};
+constexpr int32_t kPadHi = 0x7FF8DEAD;  // high word of a padding record's FP64 value (a NaN)
+
 struct CellBlockDev {
     int32_t material;
     double lambda, mu;
@@ -244,8 +254,9 @@ void launch_sensor_seed(const double4* U4, int32_t num_sensors, const int32_t* s
                         cudaStream_t s);
 
 // Layout conversion.
-void launch_rk_octets(int64_t count, int64_t num_octets, const int32_t* optr, const double2* rec, const double4* in,
-                      const int64_t* row_ptr, int64_t num_nodes, double4* out4, double* out3, cudaStream_t s);
+void launch_rk_octets(int64_t count, int64_t num_octets, const int32_t* optr, const double* w, const RowIndexDev& index,
+                      const double4* in, const int64_t* row_ptr, int64_t num_nodes, double4* out4, double* out3,
+                      cudaStream_t s);
 void launch_pack4(const double* aos3, double4* out, int64_t n, cudaStream_t s);
 void launch_unpack4(const double4* in, double* aos3, int64_t n, cudaStream_t s);
 void launch_zero4(double4* out, int64_t n, cudaStream_t s);

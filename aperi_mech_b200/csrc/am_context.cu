@@ -2335,7 +2335,7 @@ int am_adjoint(am_ctx* ctx, int64_t nsteps, double dt, int32_t ckpt_every, int32
             for (int64_t n = n1 - 1; n >= n0; --n) {
                 ctx->vjp(seg[n - n0], ctx->L4, gm, gk, 1);
                 ctx->mark(2, static_cast<int64_t>(ctx->blocks.size()));
-                am::launch_adj_update(nd, ctx->slots64, ctx->table, n, UB, VB, AB, ctx->L4, st);
+                am::launch_adj_update(nd, ctx->slots64, ctx->table, n, UB, VB, ctx->L4, st);
                 ++ctx->launches;
                 ctx->mark(3, 1);
             }

@@ -2373,85 +2373,182 @@ __global__ void __launch_bounds__(256) k_tet4_patch_vjp(GaussBlockDev b, const d
     }
 }
 
-// VJP of the Hex8 forces in the monomial basis (see k_hex8_force): the
-// Gauss point's dP[grad lam] takes the place of P in the same regrouped nodal
-// sum, and the material-field contractions are summed over the Gauss points in
-// order. One thread per element, FP64.
+// Gauss-point VJP term of a Hex8: Q = adj(J) dP^T for the stress derivative dP along
+// L = W J^-1 (J, G, W in the raw units of hex_derivatives, sig as in hex_gauss_q), and the
+// sensitivities L : dP/dlambda and L : dP/dmu at fixed H.
+// Neo-Hookean: dP^T = mu L^T + a F^-1 L F^-1 + lambda tr(F^-1 L) F^-1, a = mu - lambda log J.
+// With Jc = J + G (F = Jc J^-1) and M = J^-1 J^-T neither H, L nor F^-1 is formed:
+//   Q = det J (mu (W M)^T + a Jc^-1 W Jc^-1 + lambda tr(Jc^-1 W) Jc^-1),
+//   tr(F^-1 L) = tr(Jc^-1 W),  L : F = (W M) : Jc,
+//   J - 1 = (adj(J) : G^T + adj(G) : J^T + det G) / det J.
 template <int MAT>
-__global__ void __launch_bounds__(64) k_hex8_vjp(GaussBlockDev b, const double4* __restrict__ X4,
-                                                       const double4* __restrict__ U4, const double4* __restrict__ L4,
-                                                       double4* __restrict__ slots, double* gmu, double* gk,
-                                                       int accumulate) {
-    const int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (e >= b.num_elems) return;
-    int32_t nd[8];
-    hex_conn(b, e, nd);
-    double X[3][8], U[3][8], W[3][8];
-    hex_load_rel(X4, nd, X);
-    hex_load_rel(U4, nd, U);
-    hex_load_rel(L4, nd, W);
-#pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        hex_butterfly(X[i]);
-        hex_butterfly(U[i]);
-        hex_butterfly(W[i]);
-        hex_scale_coeffs(X[i]);
-        hex_scale_coeffs(U[i]);
-        hex_scale_coeffs(W[i]);
-    }
-    double lam, mu;
-    element_lame(b, e, lam, mu);
-    double R[3][8];
-#pragma unroll
-    for (int i = 0; i < 3; ++i)
-#pragma unroll
-        for (int k = 0; k < 8; ++k) R[i][k] = 0.0;
-    double tm = 0.0, tk = 0.0;
-#pragma unroll 1
-    for (int g = 0; g < 8; ++g) {
-        double J[9], A[9], H[9], L[9];
+__device__ __forceinline__ double hex_gauss_vjp(const double* J, const double* G, const double* W, double lam, double mu,
+                                                double* Q, double& l_dlam, double& l_dmu) {
+    double A[9];
+    adj3(J, A);
+    const double det = J[0] * A[0] + J[1] * A[3] + J[2] * A[6];
+    const double id = 1.0 / det;
+    if (MAT == kNeoHookean) {
+        double B[9], Jc[9];
+        adj3(G, B);
+        double num = G[0] * B[0] + G[1] * B[3] + G[2] * B[6];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
-            for (int j = 0; j < 3; ++j) J[i * 3 + j] = hex_dxi(X[i], j, g);
-        adj3(J, A);
-        const double det = J[0] * A[0] + J[1] * A[3] + J[2] * A[6];
-        const double id = 1.0 / det;
+            for (int j = 0; j < 3; ++j) num += A[i * 3 + j] * G[j * 3 + i] + B[i * 3 + j] * J[j * 3 + i];
+        const double lnJ = log1p_nh(num * id);
+#pragma unroll
+        for (int k = 0; k < 9; ++k) Jc[k] = J[k] + G[k];
+        adj3(Jc, B);
+        const double ic = 1.0 / (det + num);
+        double C[9], N[9], S[6];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) C[i * 3 + j] = B[i * 3 + 0] * W[0 + j] + B[i * 3 + 1] * W[3 + j] + B[i * 3 + 2] * W[6 + j];
+        const double tr = (C[0] + C[4] + C[8]) * ic;
+        // S = adj(J) adj(J)^T (upper triangle), N = W M = W S / det^2
+        S[0] = A[0] * A[0] + A[1] * A[1] + A[2] * A[2];
+        S[1] = A[0] * A[3] + A[1] * A[4] + A[2] * A[5];
+        S[2] = A[0] * A[6] + A[1] * A[7] + A[2] * A[8];
+        S[3] = A[3] * A[3] + A[4] * A[4] + A[5] * A[5];
+        S[4] = A[3] * A[6] + A[4] * A[7] + A[5] * A[8];
+        S[5] = A[6] * A[6] + A[7] * A[7] + A[8] * A[8];
+        double lf = 0.0;
 #pragma unroll
         for (int i = 0; i < 3; ++i) {
-            const double g0 = hex_dxi(U[i], 0, g), g1 = hex_dxi(U[i], 1, g), g2 = hex_dxi(U[i], 2, g);
-            const double l0 = hex_dxi(W[i], 0, g), l1 = hex_dxi(W[i], 1, g), l2 = hex_dxi(W[i], 2, g);
+            const double w0 = W[i * 3], w1 = W[i * 3 + 1], w2 = W[i * 3 + 2];
+            N[i * 3 + 0] = w0 * S[0] + w1 * S[1] + w2 * S[2];
+            N[i * 3 + 1] = w0 * S[1] + w1 * S[3] + w2 * S[4];
+            N[i * 3 + 2] = w0 * S[2] + w1 * S[4] + w2 * S[5];
 #pragma unroll
-            for (int j = 0; j < 3; ++j) {
-                H[i * 3 + j] = (g0 * A[0 * 3 + j] + g1 * A[1 * 3 + j] + g2 * A[2 * 3 + j]) * id;
-                L[i * 3 + j] = (l0 * A[0 * 3 + j] + l1 * A[1 * 3 + j] + l2 * A[2 * 3 + j]) * id;
-            }
+            for (int j = 0; j < 3; ++j) lf += N[i * 3 + j] * Jc[i * 3 + j];
         }
-        double dP[9], ldl, ldm;
-        stress_vjp(MAT, lam, mu, H, L, dP, &ldl, &ldm);
-        const double w = det * (1.0 / 512.0);
-        tm -= w * (ldm - 2.0 / 3.0 * ldl);
-        tk -= w * ldl;
-        double Q[9];
+        l_dlam = lnJ * tr;
+        l_dmu = lf * id * id - tr;
+        const double dc = det * ic, q0 = mu * id, q1 = (mu - lam * lnJ) * dc * ic, q2 = lam * tr * dc;
 #pragma unroll
         for (int k = 0; k < 3; ++k)
 #pragma unroll
-            for (int i = 0; i < 3; ++i)
-                Q[k * 3 + i] = A[k * 3 + 0] * dP[i * 3 + 0] + A[k * 3 + 1] * dP[i * 3 + 1] + A[k * 3 + 2] * dP[i * 3 + 2];
-        hex_accumulate_r(R, Q, g);
+            for (int i = 0; i < 3; ++i) {
+                const double cc = C[k * 3 + 0] * B[0 + i] + C[k * 3 + 1] * B[3 + i] + C[k * 3 + 2] * B[6 + i];
+                Q[k * 3 + i] = q0 * N[i * 3 + k] + q1 * cc + q2 * B[k * 3 + i];
+            }
+        return det;
     }
+    double H[9], L[9], dP[9];
 #pragma unroll
-    for (int i = 0; i < 3; ++i) {
-        R[i][0] = 0.0;
-        hex_scale_coeffs(R[i]);
-        hex_butterfly_t(R[i]);
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+            H[i * 3 + j] = (G[i * 3 + 0] * A[0 * 3 + j] + G[i * 3 + 1] * A[1 * 3 + j] + G[i * 3 + 2] * A[2 * 3 + j]) * id;
+            L[i * 3 + j] = (W[i * 3 + 0] * A[0 * 3 + j] + W[i * 3 + 1] * A[1 * 3 + j] + W[i * 3 + 2] * A[2 * 3 + j]) * id;
+        }
+    stress_vjp(MAT, lam, mu, H, L, dP, &l_dlam, &l_dmu);
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+            Q[k * 3 + i] = A[k * 3 + 0] * dP[i * 3 + 0] + A[k * 3 + 1] * dP[i * 3 + 1] + A[k * 3 + 2] * dP[i * 3 + 2];
+    return det;
+}
+
+// Hex8 VJP, four lanes per element as in k_hex8_force (its stages, groups and rounds); the
+// quad's lanes add their Gauss points' modulus sensitivities. On 64^3 neo-Hookean elements
+// with fields (B200): one thread per element (254 registers, spills) 117 us, quads 111 us
+// at three blocks per SM (168 registers; at four, 128 and more spills, the same; at two 128
+// us). Gather latency binds (FP64 pipe 44%).
+constexpr int kHexVjpBlocks = 3;
+template <int MAT>
+__global__ void __launch_bounds__(kHexBlock, kHexVjpBlocks) k_hex8_vjp(GaussBlockDev b, const double4* __restrict__ X4,
+                                                       const double4* __restrict__ U4, const double4* __restrict__ L4,
+                                                       double4* __restrict__ slots, double* gmu, double* gk,
+                                                       int accumulate, int32_t rounds) {
+    constexpr int NW = kHexBlock / 32;
+    const int lane = static_cast<int>(threadIdx.x & 31), p = lane & 3;
+    const int32_t E = static_cast<int32_t>(b.num_elems);
+    int32_t g = static_cast<int32_t>(blockIdx.x) * rounds * NW + static_cast<int32_t>(threadIdx.x >> 5);
+    const int32_t last = min(g + rounds * NW, (E + 7) >> 3);
+    const auto elem = [&](int32_t grp) { return min(8 * grp + (lane >> 2), E - 1); };
+    pdl_trigger();
+    if (g >= last) return;
+    int2 n = hex_edge_pair(b.conn, elem(g), p);
+    int32_t n0 = b.conn[8 * elem(g)];
+    const double sig = (p == 1 || p == 2) ? -1.0 : 1.0;
+    constexpr double s3 = kHexScale * kHexScale * kHexScale;
+    for (; g < last; g += NW) {
+        const int32_t e = elem(g);
+        HexRaw X, U, V;
+        X.load<false>(X4, n0, n);
+        double lam, mu;
+        element_lame(b, e, lam, mu);
+        const int2 pos = hex_edge_pair(b.slot_pos, e, p);
+        pdl_wait();  // at once after the first round
+        U.load<true>(U4, n0, n);
+        V.load<true>(L4, n0, n);
+        if (g + NW < last) {
+            n = hex_edge_pair(b.conn, elem(g + NW), p);
+            n0 = b.conn[8 * elem(g + NW)];
+        }
+        double J0[3], G0[3], W0[3];
+        HexPair<double> v[3], J1[3], J2[3], G1[3], G2[3], W1[3], W2[3];
+        X.rel<double>(v);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) hex_derivatives(v[i], J0[i], J1[i], J2[i]);
+        U.rel<double>(v);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) hex_derivatives(v[i], G0[i], G1[i], G2[i]);
+        V.rel<double>(v);
+#pragma unroll
+        for (int i = 0; i < 3; ++i) hex_derivatives(v[i], W0[i], W1[i], W2[i]);
+        double z[3], tm = 0.0, tk = 0.0;
+        HexPair<double> q1[3], q2[3];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            double J[9], G[9], W[9], Q[9], ldl, ldm;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                J[3 * i] = J0[i];
+                J[3 * i + 1] = h ? J1[i].b : J1[i].a;
+                J[3 * i + 2] = h ? J2[i].b : J2[i].a;
+                G[3 * i] = G0[i];
+                G[3 * i + 1] = h ? G1[i].b : G1[i].a;
+                G[3 * i + 2] = h ? G2[i].b : G2[i].a;
+                W[3 * i] = W0[i];
+                W[3 * i + 1] = h ? W1[i].b : W1[i].a;
+                W[3 * i + 2] = h ? W2[i].b : W2[i].a;
+            }
+            const double w = s3 * sig * hex_gauss_vjp<MAT>(J, G, W, lam, mu, Q, ldl, ldm);
+            tm -= w * (ldm - 2.0 / 3.0 * ldl);
+            tk -= w * ldl;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                if (h == 0) {
+                    z[i] = Q[i];
+                    q1[i].a = Q[3 + i];
+                    q2[i].a = Q[6 + i];
+                } else {
+                    z[i] += Q[i];
+                    q1[i].b = Q[3 + i];
+                    q2[i].b = Q[6 + i];
+                }
+            }
+        }
+        const bool valid = 8 * g + (lane >> 2) < E;
+        HexPair<double> f[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) f[i] = hp_scale(-s3 * sig, hex_transpose(z[i], q1[i], q2[i]));
+#pragma unroll
+        for (int m = 1; m < 4; m <<= 1) {
+            tm += __shfl_xor_sync(kFull, tm, m);
+            tk += __shfl_xor_sync(kFull, tk, m);
+        }
+        if (valid) {
+            slots[pos.x] = make4(f[0].a, f[1].a, f[2].a);
+            slots[pos.y] = make4(f[0].b, f[1].b, f[2].b);
+            if (p == 0) store_theta(gmu, gk, e, tm, tk, accumulate);
+        }
     }
-    const double s = -1.0 / 512.0;
-    const int4 p0 = reinterpret_cast<const int4*>(b.slot_pos)[2 * e], p1 = reinterpret_cast<const int4*>(b.slot_pos)[2 * e + 1];
-    const int32_t pos[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
-#pragma unroll
-    for (int q = 0; q < 8; ++q) slots[pos[hex_node_of_corner(q)]] = make4(s * R[0][q], s * R[1][q], s * R[2][q]);
-    store_theta(gmu, gk, e, tm, tk, accumulate);
 }
 
 template <int MAT>
@@ -3048,35 +3145,43 @@ __global__ void k_adj_prep(NodeDev nd, const StepParams* __restrict__ table, int
 
 // Reverse of the rest of step `step` given g = (dF/du)^T lam in the slots; then
 // prepares lam for step-1 (or for the initial acceleration when step == 0).
-__global__ void __launch_bounds__(kNodeBlock) k_adj_update(NodeDev nd, const double4* __restrict__ slots,
+// Lanes per node as the forward node kernel (node_lanes): 24.8 -> 22.5 us on 274,625 nodes
+// with eight slots each, two lanes and no store of the acceleration cotangent, which nothing
+// reads between steps.
+template <typename S, int BATCH, int LPN>
+__global__ void __launch_bounds__(kNodeBlock) k_adj_update(NodeDev nd, const vec4_t<S>* __restrict__ slots,
                                                             const StepParams* __restrict__ table, int64_t step,
                                                             double4* __restrict__ UB, double4* __restrict__ VB,
-                                                            double4* __restrict__ AB, double4* __restrict__ L4) {
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i >= nd.num_nodes) return;
+                                                            double4* __restrict__ L4) {
+    const int64_t i = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / LPN;
+    const bool own = i < nd.num_nodes;
+    const int64_t j = own ? i : 0;
+    const uint32_t w = nd.bcword[j];
+    const double m = nd.mass[j];
+    const NodeSlots q = node_slots(nd, i, own);
+    pdl_trigger();
+    pdl_wait();
+    double4 ub = ld_dep(UB + j);
+    const double4 vb = ld_dep(VB + j);
     double gx, gy, gz;
-    gather<double, 4, 1>(nd, slots, i, true, gx, gy, gz);
+    gather<S, BATCH, LPN>(nd, slots, i, own, q, gx, gy, gz);
+    if (!own || threadIdx.x % LPN != 0) return;
     const StepParams& P = table[step];
-    double4 ub = UB[i];
-    const double4 vb = VB[i];
     ub.x += gx;
     ub.y += gy;
     ub.z += gz;
-    const uint32_t w = nd.bcword[i];
     double mx, my, mz;
     free_mask(w, P.vact, mx, my, mz);
     const double wx = mx * (vb.x + P.dt * ub.x), wy = my * (vb.y + P.dt * ub.y), wz = mz * (vb.z + P.dt * ub.z);
     const double ax = P.half * wx, ay = P.half * wy, az = P.half * wz;
-    UB[i] = ub;
-    VB[i] = make_double4(wx, wy, wz, 0.0);
-    AB[i] = make_double4(ax, ay, az, 0.0);
-    const double m = nd.mass[i];
+    st4(UB + i, ub);
+    st4(VB + i, make_double4(wx, wy, wz, 0.0));
     if (step > 0) {
         const StepParams& Q = table[step - 1];
         free_mask(w, Q.aact, mx, my, mz);
-        L4[i] = make_double4(mx * (ax + Q.half * wx) / m, my * (ay + Q.half * wy) / m, mz * (az + Q.half * wz) / m, 0.0);
+        st4(L4 + i, make_double4(mx * (ax + Q.half * wx) / m, my * (ay + Q.half * wy) / m, mz * (az + Q.half * wz) / m, 0.0));
     } else {
-        L4[i] = make_double4(ax / m, ay / m, az / m, 0.0);
+        st4(L4 + i, make_double4(ax / m, ay / m, az / m, 0.0));
     }
 }
 
@@ -3714,8 +3819,9 @@ void launch_gauss_vjp(const GaussBlockDev& b, const double4* X4, const double4* 
         const unsigned grid = grid_for(b.num_elems, 256);
         AM_DISPATCH_MAT(b.material, (k_tet4_vjp<M><<<grid, 256, 0, s>>>(b, X4, U4, L4, slots, gmu, gkappa, accumulate)));
     } else {
-        const unsigned grid = grid_for(b.num_elems, 128);
-        AM_DISPATCH_MAT(b.material, (k_hex8_vjp<M><<<grid_for(b.num_elems, 64), 64, 0, s>>>(b, X4, U4, L4, slots, gmu, gkappa, accumulate)));
+        const int64_t groups = (b.num_elems + 7) / 8;
+        const int32_t rounds = hex_rounds(groups);
+        AM_DISPATCH_MAT(b.material, (launch_pdl(k_hex8_vjp<M>, grid_for(groups, rounds * (kHexBlock / 32)), kHexBlock, s, b, X4, U4, L4, slots, gmu, gkappa, accumulate, rounds)));
     }
 }
 
@@ -3933,9 +4039,10 @@ void launch_adj_prep(const NodeDev& nd, const StepParams* table, int64_t step, c
     k_adj_prep<<<grid_for(nd.num_nodes, 256), 256, 0, s>>>(nd, table, step, VB, AB, L4);
 }
 
-void launch_adj_update(const NodeDev& nd, const double4* slots, const StepParams* table, int64_t step, double4* UB,
-                       double4* VB, double4* AB, double4* L4, cudaStream_t s) {
-    k_adj_update<<<grid_for(nd.num_nodes, kNodeBlock), kNodeBlock, 0, s>>>(nd, slots, table, step, UB, VB, AB, L4);
+void launch_adj_update(const NodeDev& nd, const void* slots, const StepParams* table, int64_t step, double4* UB,
+                       double4* VB, double4* L4, cudaStream_t s) {
+    const int mixed = 0;
+    AM_NODE_DISPATCH_PDL(k_adj_update, table, step, UB, VB, L4);
 }
 
 void launch_sensor_seed(const double4* U4, int32_t num_sensors, const int32_t* sensors, double4* UB, double* loss,

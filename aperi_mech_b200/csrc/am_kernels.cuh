@@ -230,8 +230,8 @@ void launch_node_step(const NodeDev& nd, int mixed, const void* slots, const Ste
 // Adjoint node kernels.
 void launch_adj_prep(const NodeDev& nd, const StepParams* table, int64_t step, const double4* VB, const double4* AB,
                      double4* L4, cudaStream_t s);
-void launch_adj_update(const NodeDev& nd, const double4* slots, const StepParams* table, int64_t step, double4* UB,
-                       double4* VB, double4* AB, double4* L4, cudaStream_t s);
+void launch_adj_update(const NodeDev& nd, const void* slots, const StepParams* table, int64_t step, double4* UB,
+                       double4* VB, double4* L4, cudaStream_t s);
 // Power method for the stable time increment (PowerMethodProcessor.h:196-330):
 // W = U + V l eps on the free dofs (U on the prescribed ones); then
 // V = (f_eps - f_u) / (l eps m) on the free dofs (0 on the prescribed), with the

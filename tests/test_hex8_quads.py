@@ -67,3 +67,20 @@ def test_inverted_element_is_named(gpu):
         with ExplicitDynamics(coords, [Part("hex8", mat, conn=conn)]) as m:
             with pytest.raises(AmError, match=f"element/cell {int(np.nonzero((conn == far).any(axis=1))[0][0])}$"):
                 m.internal_force(u, precision)
+
+
+@pytest.mark.parametrize("dims, material", [(d, m) for d in [(1, 1, 1), (7, 1, 1), (3, 3, 1), (11, 3, 1)]
+                                            for m in ("linear_elastic", "neo_hookean", "elastic")]
+                         + [((49, 48, 49), "neo_hookean")])
+def test_vjp_group_edges(gpu, oracle_lib, dims, material):
+    """The VJP runs in the same quads and rounds: against the oracle at the parity tests' 1e-11
+    (nodal) and, for the modulus gradients, contractions of eight points whose terms cancel to
+    the strain's order (1e-3 here, so 1e-16 / 1e-3 a term and a few terms), 1e-11 of the largest."""
+    from aperi_mech_b200.model import ExplicitDynamics
+
+    coords, parts, u = _problem(dims, material, fields=dims[0] >= 11)
+    lam = np.random.default_rng(5).standard_normal(coords.shape)
+    want = oracle_lib.OracleProblem(coords, parts).vjp_force(u, lam)
+    with ExplicitDynamics(coords, parts) as m:
+        for g, w in zip(m.vjp_force(u, lam), want):
+            assert rel_err(g, w) < 1e-11

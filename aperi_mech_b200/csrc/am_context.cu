@@ -852,7 +852,9 @@ struct am_ctx {
         ++launches;
     }
 
-    void element_forces(int mixed, const double4* U) {
+    // columns false: with the coupling, the local force stays at the points (step_nodes forms
+    // Psi^T f with the update).
+    void element_forces(int mixed, const double4* U, bool columns = true) {
         void* s = slots(mixed);
         if (lagr) {
             // The semi formulation's reference configuration moved after the last step
@@ -890,9 +892,22 @@ struct am_ctx {
             nd.num_nodes = points();  // the local force lives on the points
             am::launch_gather_force4(nd, mixed, s, rk_f_local, stream);
             ++launches;
-            rk_cols(rk_f_local, rk_f);
+            if (columns) rk_cols(rk_f_local, rk_f);
         }
         check_launch("element force kernel");
+    }
+
+    // A step's force and node update on a single domain. The two-pass coupling in warp octets
+    // updates the nodes in the columns' kernel.
+    bool coupled_step() const { return rk_ptr && rkto_w; }
+    void step_nodes(int mixed, const am::NodeDev& nd, const am::StepParams* tab, int64_t n, int advance, double4* uc,
+                    int rebase) {
+        if (coupled_step())
+            am::launch_rk_step(rkto_count, rkto_ptr, rkto_w, {rkto_iptr, rkto_idx}, rk_f_local, nd, tab, n, advance, U4,
+                               V4, A4, uc, status, stream);
+        else
+            am::launch_node_step(nd, mixed, slots(mixed), tab, n, advance, U4, V4, A4, uc, status, stream, rebase);
+        ++launches;
     }
 
     // Interface exchange between the element kernels and the node kernel: each rank's
@@ -1228,15 +1243,14 @@ struct am_ctx {
     void capture_step_graph(int mixed) {
         if (!chunk_table) chunk_table = dalloc<am::StepParams>(kGraphSteps + 1, "chunk step table");
         const am::NodeDev nd = node_dev();
-        void* s = slots(mixed);
+        slots(mixed);  // allocated before the capture
         const int64_t before = launches;
         ck(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal), "begin capture");
         cudaGraph_t g = nullptr;
         try {
             for (int64_t k = 0; k < kGraphSteps; ++k) {
-                element_forces(mixed, U4);
-                am::launch_node_step(nd, mixed, s, chunk_table, k, 1, U4, V4, A4, nullptr, status, stream, 0);
-                ++launches;
+                element_forces(mixed, U4, !coupled_step());
+                step_nodes(mixed, nd, chunk_table, k, 1, nullptr, 0);
             }
         } catch (...) {
             cudaStreamEndCapture(stream, &g);
@@ -1281,7 +1295,7 @@ struct am_ctx {
             }
         }
         for (; n < n1; ++n) {
-            element_forces(mixed, U4);
+            element_forces(mixed, U4, !coupled_step());
             mark(0, static_cast<int64_t>(blocks.size()));
             const int advance = (n + 1 < n1) ? 1 : 0;
             double4* uc = (u_hist && advance) ? u_hist[n + 1 - n0] : nullptr;
@@ -1314,9 +1328,7 @@ struct am_ctx {
                 exchange(mixed);
                 mark(4, 1);
             }
-            am::launch_node_step(nd, mixed, s, table, n, advance, U4, V4, A4, uc, status, stream,
-                                 due(lagr_steps) ? 1 : 0);
-            ++launches;
+            step_nodes(mixed, nd, table, n, advance, uc, due(lagr_steps) ? 1 : 0);
             check_launch("node step kernel");
             mark(1, 1);
         }

@@ -1555,6 +1555,11 @@ __device__ __forceinline__ const float4* node_recs<float>(const CellBlockDev& b)
 template <>
 __device__ __forceinline__ const double4* node_recs<double>(const CellBlockDev& b) { return b.nrec64; }
 
+// Block size of the octet kernels. Against 256 threads (finer last waves), us a step on B200:
+// 70,785 RKPM cells mixed 48.0 -> 47.4, 384,000 F-bar subcells FP64 217 -> 211, the two-pass
+// coupling 46.3 -> 45.6; 64 threads 48.7, 211, 45.6.
+constexpr int kOctetBlock = 128;
+
 // Part k (0, 1, 2) of M_c in the component arrays of a block of E cells.
 template <typename T>
 __device__ __forceinline__ void store_cell_matrix(T* M, int64_t E, int64_t c, int k, const T (&m)[9]) {
@@ -1582,7 +1587,7 @@ __device__ __forceinline__ void load_cell_matrix(const T* M, int64_t E, int32_t 
 // gathers issued together, the next batch's records loaded while they are in flight),
 // combined over the four lanes of a cell, P(H), and M_c written by lanes k = 0, 1, 2.
 template <typename T, int MAT, int UNR, bool FBAR, int G>
-__global__ void __launch_bounds__(256) k_cell_stress(CellBlockDev b, const double4* __restrict__ U4, T* __restrict__ M,
+__global__ void __launch_bounds__(kOctetBlock) k_cell_stress(CellBlockDev b, const double4* __restrict__ U4, T* __restrict__ M,
                                                      int* status) {
     constexpr int L = 32 / G;  // lanes per cell
     pdl_trigger();
@@ -1662,7 +1667,7 @@ __global__ void __launch_bounds__(256) k_cell_stress(CellBlockDev b, const doubl
 // dual pressure as in k_fbar_fused, and M = -V P replaces H in the matrix array for the
 // node-major gather.
 template <typename T, int MAT>
-__global__ void __launch_bounds__(256) k_fbar_cell_stress(CellBlockDev b, T* __restrict__ M, int* status) {
+__global__ void __launch_bounds__(kOctetBlock) k_fbar_cell_stress(CellBlockDev b, T* __restrict__ M, int* status) {
     pdl_trigger();
     const int lane = static_cast<int>(threadIdx.x & 31);
     const int64_t g = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -1736,7 +1741,7 @@ __global__ void __launch_bounds__(256) k_fbar_cell_stress(CellBlockDev b, T* __r
 // Node octets: f = sum of M_c b over the rows in FP64 (products in the slot precision),
 // combined over the node's four lanes, written to the node's slot by lane k = 0.
 template <typename T, int UNR, int G>
-__global__ void __launch_bounds__(256) k_cell_gather(CellBlockDev b, const T* __restrict__ M, vec4_t<T>* __restrict__ slots) {
+__global__ void __launch_bounds__(kOctetBlock) k_cell_gather(CellBlockDev b, const T* __restrict__ M, vec4_t<T>* __restrict__ slots) {
     constexpr int L = 32 / G;  // lanes per node
     pdl_trigger();
     const int64_t o = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -2975,11 +2980,13 @@ __global__ void __launch_bounds__(kNodeBlock) k_gather_force4(NodeDev nd, const 
                                                                double4* __restrict__ f) {
     const int64_t i = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) / LPN;
     const bool own = i < nd.num_nodes;
-    if (LPN == 1 && !own) return;
+    const NodeSlots q = node_slots(nd, i, own);
+    pdl_trigger();
+    pdl_wait();
     double fx, fy, fz;
-    gather<S, BATCH, LPN>(nd, slots, i, own, fx, fy, fz);
+    gather<S, BATCH, LPN>(nd, slots, i, own, q, fx, fy, fz);
     if (!own || threadIdx.x % LPN != 0) return;
-    f[i] = make_double4(fx, fy, fz, 0.0);
+    st4(f + i, make_double4(fx, fy, fz, 0.0));
 }
 
 // One thread per local interface node: its own slots summed (no interface override).
@@ -3070,6 +3077,41 @@ __global__ void __launch_bounds__(256) k_prologue(NodeDev nd, const StepParams* 
     if (u_copy) u_copy[i] = u;
 }
 
+// The central-difference update of node i from its force (mass m, BC word w, half-step
+// velocity vh, displacement u0, which is read only when advance is set).
+__device__ __forceinline__ void node_update(const NodeDev& nd, int64_t i, double fx, double fy, double fz, double m, uint32_t w,
+                                            const double4& vh, const double4& u0, const StepParams* __restrict__ table,
+                                            int64_t step, int advance, double4* __restrict__ U4, double4* __restrict__ V4,
+                                            double4* __restrict__ A4, double4* __restrict__ u_copy, int* status, int rebase) {
+    if (nd.has_g) {
+        fx += nd.g[0] * m;
+        fy += nd.g[1] * m;
+        fz += nd.g[2] * m;
+    }
+    // a^{n+1} = f / m (ExplicitTimeIntegrator.h:247-283), then the acceleration BC at t^{n+1}.
+    double ax = fx / m, ay = fy / m, az = fz / m;
+    const StepParams& P = table[step];
+    if (w) apply_bc(w, P.aact, P.ascale, nd.bcvalues, ax, ay, az);
+    if (!isfinite(ax) || !isfinite(ay) || !isfinite(az)) flag(status, AM_ENAN, i);
+    // v^{n+1} = v^{n+1/2} + dt/2 a^{n+1} (:329-364)
+    const double vx = vh.x + P.half * ax, vy = vh.y + P.half * ay, vz = vh.z + P.half * az;
+    if (advance) {
+        // Next step: v^{n+3/2} = v^{n+1} + dt'/2 a^{n+1} (:286-326), velocity BC at t_mid',
+        // u^{n+2} = u^{n+1} + dt' v^{n+3/2} (:97-134).
+        const StepParams& Q = table[step + 1];
+        double wx = vx + Q.half * ax, wy = vy + Q.half * ay, wz = vz + Q.half * az;
+        if (w) apply_bc(w, Q.vact, Q.vscale, nd.bcvalues, wx, wy, wz);
+        double4 u = u0;
+        displace(nd, i, rebase, Q.dt, wx, wy, wz, u);
+        st4(U4 + i, u);
+        st4(V4 + i, make_double4(wx, wy, wz, 0.0));
+        if (u_copy) st4(u_copy + i, u);
+    } else {
+        st4(V4 + i, make_double4(vx, vy, vz, 0.0));
+        st4(A4 + i, make_double4(ax, ay, az, 0.0));
+    }
+}
+
 template <typename S, int BATCH, int LPN>
 __global__ void __launch_bounds__(kNodeBlock) k_node_step(NodeDev nd, const vec4_t<S>* __restrict__ slots,
                                                            const StepParams* __restrict__ table, int64_t step,
@@ -3099,33 +3141,7 @@ __global__ void __launch_bounds__(kNodeBlock) k_node_step(NodeDev nd, const vec4
     double fx, fy, fz;
     gather<S, BATCH, LPN>(nd, slots, i, own, q, fx, fy, fz);
     if (!own || threadIdx.x % LPN != 0) return;
-    if (nd.has_g) {
-        fx += nd.g[0] * m;
-        fy += nd.g[1] * m;
-        fz += nd.g[2] * m;
-    }
-    // a^{n+1} = f / m (ExplicitTimeIntegrator.h:247-283), then the acceleration BC at t^{n+1}.
-    double ax = fx / m, ay = fy / m, az = fz / m;
-    const StepParams& P = table[step];
-    if (w) apply_bc(w, P.aact, P.ascale, nd.bcvalues, ax, ay, az);
-    if (!isfinite(ax) || !isfinite(ay) || !isfinite(az)) flag(status, AM_ENAN, i);
-    // v^{n+1} = v^{n+1/2} + dt/2 a^{n+1} (:329-364)
-    const double vx = vh.x + P.half * ax, vy = vh.y + P.half * ay, vz = vh.z + P.half * az;
-    if (advance) {
-        // Next step: v^{n+3/2} = v^{n+1} + dt'/2 a^{n+1} (:286-326), velocity BC at t_mid',
-        // u^{n+2} = u^{n+1} + dt' v^{n+3/2} (:97-134).
-        const StepParams& Q = table[step + 1];
-        double wx = vx + Q.half * ax, wy = vy + Q.half * ay, wz = vz + Q.half * az;
-        if (w) apply_bc(w, Q.vact, Q.vscale, nd.bcvalues, wx, wy, wz);
-        double4 u = u0;
-        displace(nd, i, rebase, Q.dt, wx, wy, wz, u);
-        st4(U4 + i, u);
-        st4(V4 + i, make_double4(wx, wy, wz, 0.0));
-        if (u_copy) st4(u_copy + i, u);
-    } else {
-        st4(V4 + i, make_double4(vx, vy, vz, 0.0));
-        st4(A4 + i, make_double4(ax, ay, az, 0.0));
-    }
+    node_update(nd, i, fx, fy, fz, m, w, vh, u0, table, step, advance, U4, V4, A4, u_copy, status, rebase);
 }
 
 // Reverse of the acceleration step: lam = Ma (abar + h vbar) / m, the cotangent
@@ -3338,15 +3354,27 @@ __global__ void __launch_bounds__(128) k_rk_cols3(int64_t n, const int64_t* __re
 // octet's rows are aligned by offset (a quarter-warp's eight gathers then read consecutive
 // nodes or points), one index key: 8.5 bytes per record instead of 16 with the index beside
 // the weight. Rows of Psi without neighbours copy the node's coefficient (out4 set, row_ptr
-// the original offsets); columns write out3. On 70,785 nodes (32 x 32 x 64 box, B200) the two
+// the original offsets); columns write out3 or (STEP) advance the node by the force they
+// formed, in place of a node kernel. On 70,785 nodes (32 x 32 x 64 box, B200) the two
 // coupling launches of a step read 39 -> 24 MB each and took 17.5 -> 15.2 us; latency of the
-// gathers binds now.
-template <int UNR>
-__global__ void __launch_bounds__(256) k_rk_octets(int64_t count, int64_t num_octets, const int32_t* __restrict__ optr,
+// gathers binds now. Programmatic launches of the step's kernels and the node update in the
+// columns: 53.7 -> 45.6 us a step.
+struct NodeStepArgs {
+    NodeDev nd;
+    const StepParams* table;
+    int64_t step;
+    int32_t advance;
+    double4 *U4, *V4, *A4, *u_copy;
+    int* status;
+};
+template <int UNR, bool STEP>
+__global__ void __launch_bounds__(kOctetBlock) k_rk_octets(int64_t count, int64_t num_octets, const int32_t* __restrict__ optr,
                                                    const double* __restrict__ w, RowIndexDev index,
                                                    const double4* __restrict__ in,
                                                    const int64_t* __restrict__ row_ptr, int64_t num_nodes,
-                                                   double4* __restrict__ out4, double* __restrict__ out3) {
+                                                   double4* __restrict__ out4, double* __restrict__ out3,
+                                                   NodeStepArgs a) {
+    pdl_trigger();
     const int64_t o = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     const int lane = static_cast<int>(threadIdx.x & 31), j = lane & 7, k = lane >> 3;
     const int64_t i = 8 * o + j;
@@ -3370,6 +3398,19 @@ __global__ void __launch_bounds__(256) k_rk_octets(int64_t count, int64_t num_oc
     double2 rr[UNR];
 #pragma unroll
     for (int u = 0; u < UNR; ++u) rr[u] = k + 4 * u < rows ? row(k + 4 * u) : pad;
+    const bool mine = valid && k == 0;
+    double m = 1.0;
+    uint32_t bc = 0;
+    double4 vh{}, u0{};
+    if (STEP && mine) {
+        m = a.nd.mass[i];
+        bc = a.nd.bcword[i];
+    }
+    pdl_wait();
+    if (STEP && mine) {
+        vh = ld_dep(a.V4 + i);
+        if (a.advance) u0 = ld_dep(a.U4 + i);
+    }
     double x = 0.0, y = 0.0, z = 0.0;
 #pragma unroll 1
     for (int32_t r = k; r < rows; r += 4 * UNR) {
@@ -3377,7 +3418,7 @@ __global__ void __launch_bounds__(256) k_rk_octets(int64_t count, int64_t num_oc
 #pragma unroll
         for (int u = 0; u < UNR; ++u) {
             const int32_t idx = static_cast<int32_t>(__double_as_longlong(rr[u].y));
-            g[u] = idx >= 0 ? ld_ro4(in + idx) : make_double4(0.0, 0.0, 0.0, 0.0);
+            g[u] = idx >= 0 ? ld_dep(in + idx) : make_double4(0.0, 0.0, 0.0, 0.0);
         }
         double2 nx[UNR];
 #pragma unroll
@@ -3400,11 +3441,13 @@ __global__ void __launch_bounds__(256) k_rk_octets(int64_t count, int64_t num_oc
         y += __shfl_xor_sync(kFull, y, off);
         z += __shfl_xor_sync(kFull, z, off);
     }
-    if (!valid || k != 0) return;
-    if (out4 != nullptr) {
-        out4[i] = row_ptr[i + 1] != row_ptr[i] ? make_double4(x, y, z, 0.0)
-                  : i < num_nodes              ? in[i]
-                                               : make_double4(0.0, 0.0, 0.0, 0.0);
+    if (!mine) return;
+    if (STEP) {
+        node_update(a.nd, i, x, y, z, m, bc, vh, u0, a.table, a.step, a.advance, a.U4, a.V4, a.A4, a.u_copy, a.status, 0);
+    } else if (out4 != nullptr) {
+        st4(out4 + i, row_ptr[i + 1] != row_ptr[i] ? make_double4(x, y, z, 0.0)
+                      : i < num_nodes              ? ld_dep(in + i)
+                                                   : make_double4(0.0, 0.0, 0.0, 0.0));
     } else {
         out3[3 * i] = x;
         out3[3 * i + 1] = y;
@@ -3691,13 +3734,13 @@ template <typename T, int UNR, int G>
 void launch_cell_stress_g(const CellBlockDev& b, const double4* U4, int* status, cudaStream_t s) {
     if (b.group_ptr != nullptr) {
         // F-bar: H per subcell, then M per cell of subcells
-        launch_pdl(k_cell_stress<T, kLinearElastic, UNR, true, G>, grid_for(b.num_octets * 32, 256), 256, s, b, U4,
+        launch_pdl(k_cell_stress<T, kLinearElastic, UNR, true, G>, grid_for(b.num_octets * 32, kOctetBlock), kOctetBlock, s, b, U4,
                    static_cast<T*>(b.cmat), status);
-        AM_DISPATCH_MAT(b.material, (launch_pdl(k_fbar_cell_stress<T, M>, grid_for(b.num_groups * 32, 256), 256, s, b,
+        AM_DISPATCH_MAT(b.material, (launch_pdl(k_fbar_cell_stress<T, M>, grid_for(b.num_groups * 32, kOctetBlock), kOctetBlock, s, b,
                                                 static_cast<T*>(b.cmat), status)));
         return;
     }
-    AM_DISPATCH_MAT(b.material, (launch_pdl(k_cell_stress<T, M, UNR, false, G>, grid_for(b.num_octets * 32, 256), 256, s, b,
+    AM_DISPATCH_MAT(b.material, (launch_pdl(k_cell_stress<T, M, UNR, false, G>, grid_for(b.num_octets * 32, kOctetBlock), kOctetBlock, s, b,
                                             U4, static_cast<T*>(b.cmat), status)));
 }
 template <typename T, int UNR>
@@ -3710,10 +3753,10 @@ void launch_cell_stress_unr(const CellBlockDev& b, const double4* U4, int* statu
 template <typename T, int UNR>
 void launch_cell_gather_unr(const CellBlockDev& b, void* slots, cudaStream_t s) {
     if (b.group_items[1] == 1)
-        launch_pdl(k_cell_gather<T, UNR, 1>, grid_for(b.num_node_octets * 32, 256), 256, s, b, static_cast<const T*>(b.cmat),
+        launch_pdl(k_cell_gather<T, UNR, 1>, grid_for(b.num_node_octets * 32, kOctetBlock), kOctetBlock, s, b, static_cast<const T*>(b.cmat),
                    static_cast<vec4_t<T>*>(slots));
     else
-        launch_pdl(k_cell_gather<T, UNR, 8>, grid_for(b.num_node_octets * 32, 256), 256, s, b, static_cast<const T*>(b.cmat),
+        launch_pdl(k_cell_gather<T, UNR, 8>, grid_for(b.num_node_octets * 32, kOctetBlock), kOctetBlock, s, b, static_cast<const T*>(b.cmat),
                    static_cast<vec4_t<T>*>(slots));
 }
 // Rows in flight per lane: unroll[0] (cell kernel) and unroll[1] (gather kernel), 1, 2 or 4.
@@ -3830,11 +3873,11 @@ void launch_gauss_vjp(const GaussBlockDev& b, const double4* X4, const double4* 
 template <int UNR, int G>
 void launch_fbar_vjp_g(const CellBlockDev& b, const double4* U4, const double4* L4, double* Lm, double* gmu,
                        double* gkappa, int accumulate, cudaStream_t s) {
-    const unsigned grid = grid_for(b.num_octets * 32, 256);
+    const unsigned grid = grid_for(b.num_octets * 32, kOctetBlock);
     double* Hm = static_cast<double*>(b.cmat);
     // the H-only instance returns before any status flag
-    launch_pdl(k_cell_stress<double, kLinearElastic, UNR, true, G>, grid, 256, s, b, U4, Hm, static_cast<int*>(nullptr));
-    launch_pdl(k_cell_stress<double, kLinearElastic, UNR, true, G>, grid, 256, s, b, L4, Lm, static_cast<int*>(nullptr));
+    launch_pdl(k_cell_stress<double, kLinearElastic, UNR, true, G>, grid, kOctetBlock, s, b, U4, Hm, static_cast<int*>(nullptr));
+    launch_pdl(k_cell_stress<double, kLinearElastic, UNR, true, G>, grid, kOctetBlock, s, b, L4, Lm, static_cast<int*>(nullptr));
     AM_DISPATCH_MAT(b.material, (launch_pdl(k_fbar_cell_vjp<M>, grid_for(b.num_groups * 32, 256), 256, s, b, Hm,
                                             static_cast<const double*>(Lm), gmu, gkappa, accumulate)));
 }
@@ -3996,7 +4039,7 @@ void launch_gather_force(const NodeDev& nd, int mixed, const void* slots, double
     AM_NODE_DISPATCH(k_gather_force, f, accumulate);
 }
 void launch_gather_force4(const NodeDev& nd, int mixed, const void* slots, double4* f, cudaStream_t s) {
-    AM_NODE_DISPATCH(k_gather_force4, f);
+    AM_NODE_DISPATCH_PDL(k_gather_force4, f);
 }
 
 void launch_iface_gather(const NodeDev& nd, int mixed, const void* slots, int64_t num_local,
@@ -4090,8 +4133,15 @@ void launch_rk_octets(int64_t count, int64_t num_octets, const int32_t* optr, co
                       const double4* in, const int64_t* row_ptr, int64_t num_nodes, double4* out4, double* out3,
                       cudaStream_t s) {
     if (count > 0)
-        k_rk_octets<4><<<grid_for(num_octets * 32, 256), 256, 0, s>>>(count, num_octets, optr, w, index, in, row_ptr,
-                                                                      num_nodes, out4, out3);
+        launch_pdl(k_rk_octets<4, false>, grid_for(num_octets * 32, kOctetBlock), kOctetBlock, s, count, num_octets, optr, w, index, in,
+                   row_ptr, num_nodes, out4, out3, NodeStepArgs{});
+}
+void launch_rk_step(int64_t num_octets, const int32_t* optr, const double* w, const RowIndexDev& index, const double4* in,
+                    const NodeDev& nd, const StepParams* table, int64_t step, int advance, double4* U4, double4* V4,
+                    double4* A4, double4* u_copy, int* status, cudaStream_t s) {
+    launch_pdl(k_rk_octets<4, true>, grid_for(num_octets * 32, kOctetBlock), kOctetBlock, s, nd.num_nodes, num_octets, optr, w, index, in,
+               nullptr, nd.num_nodes, nullptr, nullptr,
+               NodeStepArgs{nd, table, step, advance, U4, V4, A4, u_copy, status});
 }
 
 void launch_pack4(const double* aos3, double4* out, int64_t n, cudaStream_t s) {

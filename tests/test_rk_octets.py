@@ -48,3 +48,41 @@ def test_coupled_force_matches_oracle(gpu, oracle_lib, dims, kind):
     want = oracle_lib.OracleProblem(coords, [part], mass=mass, rk=rk)
     with ExplicitDynamics(coords, [part], mass=mass, rk=rk) as m:
         assert rel_err(m.internal_force(d, "fp64"), want.internal_force(d)) < 1e-12
+
+
+@pytest.mark.parametrize("octets", ["1", "0"])
+@pytest.mark.parametrize("dims", [(2, 2, 1), (6, 5, 4)])
+def test_coupled_steps_match_oracle(gpu, oracle_lib, monkeypatch, dims, octets):
+    """Steps whose nodes the columns' kernel advances (and, with the octets off, the node
+    kernel), one at a time and 40 in a run (past the first graph replay), with a held face and
+    gravity, against the oracle's steps: u and v at the parity tests' 1e-12, the acceleration, a
+    residual of larger stresses, at 1e-11 as in the full-size tests."""
+    from aperi_mech_b200 import mesh
+    from aperi_mech_b200.model import BoundaryCondition, ExplicitDynamics, Material
+    from aperi_mech_b200.smoothing import element_smoothing_part
+
+    monkeypatch.setenv("APERI_B200_RK_OCTETS", octets)
+    rng = np.random.default_rng(sum(dims))
+    coords, hexes = mesh.box_hex(*dims)
+    conn = mesh.hex_to_tets(hexes)
+    mat = Material.create("neo_hookean", 1000.0, shear_modulus=3.85e8, bulk_modulus=8.33e8)
+    part, mass = element_smoothing_part(coords, conn, mat)
+    ptr, nbr, val = _functions(coords.shape[0], "mixed", rng)
+    val = np.where(val == 0.0, 0.0, 0.05 * val)  # weak coupling: the step stays stable
+    bcs = [BoundaryCondition.fixed(mesh.side_sets(coords)["surface_5"])]
+    v0 = rng.uniform(-0.1, 0.1, coords.shape)
+    v0[bcs[0].nodes] = 0.0
+    dt = 0.2 * float(mesh.tet_char_length(coords, conn).min()) / np.sqrt((mat.lam + 2 * mat.mu) / 1000.0)
+    g = (0.0, 0.3, -9.81)
+    z = np.zeros_like(coords)
+    op = oracle_lib.OracleProblem(coords, [part], bcs, mass=mass, body_accel=g, rk=(ptr, nbr, val))
+    a0 = op.init_acceleration(z)
+    with ExplicitDynamics(coords, [part], bcs, body_accel=g, mass=mass, rk=(ptr, nbr, val)) as m:
+        for runs in ([3], [1, 1, 1], [40], [40]):
+            want = op.steps(z, v0, a0, np.full(sum(runs), dt))
+            m.set_state(z, v0)
+            m.init_acceleration()
+            for k, r in enumerate(runs):
+                m.run(r, dt, t0=sum(runs[:k]) * dt)
+            for got, ref, tol in zip(m.get_state(), want, (1e-12, 1e-12, 1e-11)):
+                assert rel_err(got, ref) < tol

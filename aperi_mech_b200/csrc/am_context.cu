@@ -223,7 +223,9 @@ struct Block {
     int32_t* cell_ptr = nullptr;
     int32_t* cell_nodes = nullptr;
     double* grads64 = nullptr;
-    float* grads32 = nullptr;
+    float* grads32 = nullptr;   // not kept where unit32 is
+    float* unit32 = nullptr;    // half-patch tables of grouped four-entry cells (see CellBlockDev)
+    double* unit64 = nullptr;
     double* volumes = nullptr;
     int32_t max_entries = 0;
     // Updated / semi-Lagrangian state (am_set_formulation): H of the last force evaluation
@@ -364,6 +366,8 @@ struct Block {
         c.nodes = cell_nodes;
         c.grads64 = grads64;
         c.grads32 = grads32;
+        c.unit32 = unit32;
+        c.unit64 = unit64;
         c.volumes = volumes;
         c.mu_field = mu_field;
         c.kappa_field = kappa_field;
@@ -429,6 +433,8 @@ struct Block {
         dfree(cell_nodes);
         dfree(grads64);
         dfree(grads32);
+        dfree(unit32);
+        dfree(unit64);
         dfree(volumes);
         dfree(patch_first);
         dfree(patch_nodes);
@@ -879,7 +885,7 @@ struct am_ctx {
         }
         for (auto& b : blocks) {
             if (b.kind == AM_SMOOTHED_CELLS) {
-                if (mixed && !b.grads32) fail(AM_ESTATE, "mixed precision needs FP32 cell gradients");
+                if (mixed && !b.grads32 && !b.unit32) fail(AM_ESTATE, "mixed precision needs FP32 cell gradients");
                 launches += am::launch_cell_force(b.cells_for(mixed), mixed, U, s, status, stream);
             } else {
                 am::launch_gauss_force(b.gauss(), mixed, X4, U, s, status, stream);
@@ -1697,6 +1703,11 @@ int am_add_block(am_ctx* ctx, const am_block_desc* d, int32_t* block_id) {
                         ck(cudaMemcpy(b.patch_first, tp.first.data(), (P + 1) * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
                         ck(cudaMemcpy(b.patch_nodes, tp.nodes.data(), 8 * P * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
                         b.host_nodes.assign(tp.nodes.begin(), tp.nodes.begin() + 8 * P);
+                        dfree(b.grads32);
+                        b.unit32 = dalloc<float>(80 * P, "half-patch gradients (FP32)");
+                        b.unit64 = dalloc<double>(80 * P, "half-patch gradients");
+                        am::launch_cell_units(b.grads64, b.volumes, P, b.unit32, b.unit64, ctx->stream);
+                        ck(cudaGetLastError(), "half-patch gradients");
                         if (ctx->warp_chunks && ctx->lagr == 0) {
                             // warp chunks over the half patches, as for the split-hex tets
                             constexpr int kNode[2][4] = {{1, 2, 4, 0}, {5, 6, 7, 3}};

@@ -63,6 +63,59 @@ __device__ __forceinline__ double4 ld_ro4(const double4* p) {
 // Sends a line that is read later (past other loads' latency) to L2.
 __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); }
 
+// Loads of run-invariant data that a kernel reads once (connectivity, tables, plans): the
+// read-only path without an L1 line, which the nodal gathers beside them then keep. On B200,
+// us a step: smoothed cells of the h = 1/46 box mixed 33.2 -> 30.6, 128^3 Hex8 mixed 397 ->
+// 389, renumbered tets FP64 50.7 -> 49.1, 50 adjoint steps of 64^3 Hex8 15.1 -> 14.5 ms.
+// Not for sectors that two loads share (patch nodes, reference differences): 30.6 -> 31.7 and,
+// split-hex tets mixed, 47.4 -> 47.6.
+__device__ __forceinline__ int32_t ld_once(const int32_t* p) {
+    int32_t r;
+    asm("ld.global.nc.L1::no_allocate.s32 %0, [%1];" : "=r"(r) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ uint32_t ld_once(const uint32_t* p) { return static_cast<uint32_t>(ld_once(reinterpret_cast<const int32_t*>(p))); }
+__device__ __forceinline__ int2 ld_once(const int2* p) {
+    int2 r;
+    asm("ld.global.nc.L1::no_allocate.v2.s32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ int4 ld_once(const int4* p) {
+    int4 r;
+    asm("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];" : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ float ld_once(const float* p) {
+    float r;
+    asm("ld.global.nc.L1::no_allocate.f32 %0, [%1];" : "=f"(r) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ float2 ld_once(const float2* p) {
+    float2 r;
+    asm("ld.global.nc.L1::no_allocate.v2.f32 {%0, %1}, [%2];" : "=f"(r.x), "=f"(r.y) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ float4 ld_once(const float4* p) {
+    float4 r;
+    asm("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ double ld_once(const double* p) {
+    double r;
+    asm("ld.global.nc.L1::no_allocate.f64 %0, [%1];" : "=d"(r) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ double2 ld_once(const double2* p) {
+    double2 r;
+    asm("ld.global.nc.L1::no_allocate.v2.f64 {%0, %1}, [%2];" : "=d"(r.x), "=d"(r.y) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ double4 ld_once(const double4* p) {
+    double4 r;
+    asm("ld.global.nc.L1::no_allocate.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(r.x), "=d"(r.y), "=d"(r.z), "=d"(r.w) : "l"(p));
+    return r;
+}
+
 __device__ __forceinline__ void flag(int* status, int code, int64_t idx) {
     if (status == nullptr) return;
     if (atomicCAS(status + kStatusCode, 0, code) == 0) status[kStatusIndex] = static_cast<int>(idx);
@@ -222,8 +275,6 @@ template <>
 __device__ __forceinline__ const float* tet_geo<float>(const GaussBlockDev& b) { return b.geo32; }
 template <>
 __device__ __forceinline__ const double* tet_geo<double>(const GaussBlockDev& b) { return b.geo64; }
-__device__ __forceinline__ float4 ld_geo4(const float4* p) { return __ldg(p); }
-__device__ __forceinline__ double4 ld_geo4(const double4* p) { return ld_ro4(p); }
 
 __global__ void __launch_bounds__(256) k_tet4_geometry(const int32_t* __restrict__ conn, int64_t E,
                                                         const double4* __restrict__ X4, float* __restrict__ g32,
@@ -271,9 +322,9 @@ __device__ __forceinline__ ChunkLane<K> chunk_lane(const B& b, int64_t ch, int l
         const int64_t l = 32 * ch + lane;
 #pragma unroll
         for (int w = 0; w < W; ++w) {
-            L.cw[w] = b.chunk_code[l * W + w];
-            L.rw[w] = b.chunk_rank[l * W + w];
-            const int4 p = reinterpret_cast<const int4*>(b.chunk_pos)[l * W + w];
+            L.cw[w] = ld_once(b.chunk_code + l * W + w);
+            L.rw[w] = ld_once(b.chunk_rank + l * W + w);
+            const int4 p = ld_once(reinterpret_cast<const int4*>(b.chunk_pos) + l * W + w);
             L.pos[4 * w] = p.x, L.pos[4 * w + 1] = p.y, L.pos[4 * w + 2] = p.z, L.pos[4 * w + 3] = p.w;
         }
     }
@@ -376,11 +427,11 @@ __global__ void __launch_bounds__(256, CHUNKS && sizeof(T) == 8 ? 3 : 0) k_tet4_
     // chunked: lanes past the last tet run a copy of it (never summed) to reach the warp sum
     if (!CHUNKS && et >= E) return;
     const int64_t e = et < E ? et : E - 1;
-    const int4 c = reinterpret_cast<const int4*>(b.conn)[e];
+    const int4 c = ld_once(reinterpret_cast<const int4*>(b.conn) + e);
     const T* geo = tet_geo<T>(b);
-    const vec4_t<T> g0 = ld_geo4(reinterpret_cast<const vec4_t<T>*>(geo) + e);
-    const vec4_t<T> g1 = ld_geo4(reinterpret_cast<const vec4_t<T>*>(geo + 4 * E) + e);
-    const typename Vec2Of<T>::type g2 = __ldg(reinterpret_cast<const typename Vec2Of<T>::type*>(geo + 8 * E) + e);
+    const vec4_t<T> g0 = ld_once(reinterpret_cast<const vec4_t<T>*>(geo) + e);
+    const vec4_t<T> g1 = ld_once(reinterpret_cast<const vec4_t<T>*>(geo + 4 * E) + e);
+    const typename Vec2Of<T>::type g2 = ld_once(reinterpret_cast<const typename Vec2Of<T>::type*>(geo + 8 * E) + e);
     int32_t pos[4] = {0, 0, 0, 0};
     const int64_t ch = et >> 5;
     const int lane = static_cast<int>(threadIdx.x & 31);
@@ -654,7 +705,7 @@ __global__ void __launch_bounds__(kHex6Block, hex6_min_blocks<T>()) k_tet4_hex6_
     T acc0[3] = {T(0), T(0), T(0)}, acc3[3] = {T(0), T(0), T(0)}, accr[4][3];
 #pragma unroll
     for (int k = 0; k < 4; ++k) accr[k][0] = accr[k][1] = accr[k][2] = T(0);
-    const int64_t e0 = static_cast<int64_t>(b.patch_first[pp]) + 3 * r;
+    const int64_t e0 = 6 * pp + 3 * r;  // a split-hex patch holds six consecutive tets
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         // columns of J and D: X_l - X_0 and u_l - u_0 for l = R_r[k], R_r[k+1], 3
@@ -1016,7 +1067,7 @@ __device__ __forceinline__ bool hex_gauss_q(const V* J, const V* G, double lam, 
 // The two nodes of corners 2p, 2p + 1 of element e from a per-node table (nodes (0,1), (3,2),
 // (4,5), (7,6)).
 __device__ __forceinline__ int2 hex_edge_pair(const int32_t* per_node, int64_t e, int p) {
-    const int2 q = reinterpret_cast<const int2*>(per_node)[4 * e + p];
+    const int2 q = ld_once(reinterpret_cast<const int2*>(per_node) + 4 * e + p);
     return p & 1 ? make_int2(q.y, q.x) : q;
 }
 
@@ -1064,10 +1115,11 @@ __global__ void __launch_bounds__(kHexBlock, hex_min_blocks<T>()) k_hex8_force(G
     pdl_trigger();
     if (g >= last) return;
     int2 n = hex_edge_pair(b.conn, elem(g), p);
-    int32_t n0 = b.conn[8 * elem(g)];
     const double sig = (p == 1 || p == 2) ? -1.0 : 1.0;
     for (; g < last; g += W) {
         const int32_t e = elem(g);
+        // node 0: the first corner of the quad's first lane
+        const int32_t n0 = __shfl_sync(kFull, n.x, lane & ~3);
         HexRaw X, U;
         X.load<false>(X4, n0, n);
         double lam, mu;
@@ -1076,10 +1128,7 @@ __global__ void __launch_bounds__(kHexBlock, hex_min_blocks<T>()) k_hex8_force(G
         pdl_wait();  // at once after the first round
         U.load<true>(U4, n0, n);
         // the next group's connectivity travels while this one is computed
-        if (g + W < last) {
-            n = hex_edge_pair(b.conn, elem(g + W), p);
-            n0 = b.conn[8 * elem(g + W)];
-        }
+        if (g + W < last) n = hex_edge_pair(b.conn, elem(g + W), p);
         HexPair<T> x[3], u[3];
         X.rel<T>(x);
         U.rel<T>(u);
@@ -1222,7 +1271,7 @@ __global__ void __launch_bounds__(128, 5) k_tet4_force_lagr(GaussBlockDev b, int
     if (!CHUNKS && et >= E) return;
     const bool own = et < E;
     const int64_t e = own ? et : E - 1;
-    const int4 c = reinterpret_cast<const int4*>(b.conn)[e];
+    const int4 c = ld_once(reinterpret_cast<const int4*>(b.conn) + e);
     int32_t pos[4] = {0, 0, 0, 0};
     if (CHUNKS) {
         prefetch_l2(b.chunk_code + e);
@@ -1801,30 +1850,28 @@ __global__ void __launch_bounds__(kOctetBlock) k_cell_gather(CellBlockDev b, con
 // forces -V b_e P^T are summed per patch node and written to its slot.
 // ---------------------------------------------------------------------------
 template <typename T>
-__device__ __forceinline__ void load_cell12(const T* p, T* g);
+__device__ __forceinline__ const vec4_t<T>* cell_units(const CellBlockDev& b);
 template <>
-__device__ __forceinline__ void load_cell12<float>(const float* p, float* g) {
-    const float4* q = reinterpret_cast<const float4*>(p);
-#pragma unroll
-    for (int k = 0; k < 3; ++k) {
-        const float4 v = __ldg(q + k);
-        g[4 * k] = v.x;
-        g[4 * k + 1] = v.y;
-        g[4 * k + 2] = v.z;
-        g[4 * k + 3] = v.w;
-    }
-}
+__device__ __forceinline__ const float4* cell_units<float>(const CellBlockDev& b) { return reinterpret_cast<const float4*>(b.unit32); }
 template <>
-__device__ __forceinline__ void load_cell12<double>(const double* p, double* g) {
-    const double2* q = reinterpret_cast<const double2*>(p);
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        const double2 v = __ldg(q + k);
-        g[2 * k] = v.x;
-        g[2 * k + 1] = v.y;
-    }
+__device__ __forceinline__ const double4* cell_units<double>(const CellBlockDev& b) { return reinterpret_cast<const double4*>(b.unit64); }
+
+// Set-up: the half-patch tables from the cells' CSR (CellBlockDev::unit32, unit64).
+__global__ void __launch_bounds__(256) k_cell_units(const double* __restrict__ grads, const double* __restrict__ volumes,
+                                                    int64_t units, float4* __restrict__ u32, double4* __restrict__ u64) {
+    const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    const int64_t m = t / units, u = t % units;
+    if (m >= 10) return;
+    const double* g = m < 9 ? grads + 36 * u + 4 * m : volumes + 3 * u;
+    const double4 v = make_double4(g[0], g[1], g[2], m < 9 ? g[3] : 0.0);
+    u64[m * units + u] = v;
+    u32[m * units + u] = make_float4(static_cast<float>(v.x), static_cast<float>(v.y), static_cast<float>(v.z), static_cast<float>(v.w));
 }
 
+// Gradients and volumes come from the half-patch tables, whose vec4 loads are contiguous over
+// a warp (from the cells' own rows a lane's loads lay 144 bytes apart): h = 1/46 box mixed
+// 35.3 -> 33.0 us a step, and 30.6 with the tables kept out of L1. Bound: 97 MB of tables,
+// plans and slots at 55% of the measured HBM rate, latency of the u gathers.
 template <typename T, int MAT, bool CHUNKS>
 __global__ void __launch_bounds__(kHex6Block, hex6_min_blocks<T>()) k_cell_hex6_force(CellBlockDev b, const double4* U4,
                                                                                     vec4_t<T>* slots, int* status) {
@@ -1850,7 +1897,9 @@ __global__ void __launch_bounds__(kHex6Block, hex6_min_blocks<T>()) k_cell_hex6_
     nr[1] = r ? hi.z : lo.z;
     nr[2] = r ? hi.w : hi.x;
     nr[3] = r ? lo.y : hi.y;
-    const int64_t c0 = static_cast<int64_t>(b.patch_first[pp]) + 3 * r;
+    const int64_t c0 = 6 * pp + 3 * r;  // a split-hex patch holds six consecutive cells
+    const int64_t units = 2 * b.num_patches;
+    const vec4_t<T>* ut = cell_units<T>(b) + 2 * pp + r;
     pdl_trigger();
     pdl_wait();
     T du3[3], dur[4][3];
@@ -1871,12 +1920,13 @@ __global__ void __launch_bounds__(kHex6Block, hex6_min_blocks<T>()) k_cell_hex6_
     T acc0[3] = {T(0), T(0), T(0)}, acc3[3] = {T(0), T(0), T(0)}, accr[4][3];
 #pragma unroll
     for (int k = 0; k < 4; ++k) accr[k][0] = accr[k][1] = accr[k][2] = T(0);
-    const T* gr = cell_grads<T>(b);
+    const vec4_t<T> vols = ld_once(ut + 9 * units);
 #pragma unroll
     for (int k = 0; k < 3; ++k) {
         const int64_t c = c0 + k;
-        T g[12];  // b_e for the entries on local nodes 0, R_r[k], R_r[k+1], 3
-        load_cell12<T>(gr + 12 * c, g);
+        // b_e for the entries on local nodes 0, R_r[k], R_r[k+1], 3
+        const vec4_t<T> ga = ld_once(ut + (3 * k) * units), gb = ld_once(ut + (3 * k + 1) * units), gc = ld_once(ut + (3 * k + 2) * units);
+        const T g[12] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w, gc.x, gc.y, gc.z, gc.w};
         T H[9];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
@@ -1887,7 +1937,7 @@ __global__ void __launch_bounds__(kHex6Block, hex6_min_blocks<T>()) k_cell_hex6_
         T P[9];
         const double Jf = stress<T>(MAT, T(lam), T(mu), H, P);
         if (valid && MAT == kNeoHookean && !(Jf > 0.0)) flag(status, AM_ENONPOS_J, c);
-        const T V = T(b.volumes[c]);
+        const T V = k == 0 ? vols.x : k == 1 ? vols.y : vols.z;
         T f[4][3];
 #pragma unroll
         for (int e = 0; e < 4; ++e)
@@ -2478,11 +2528,11 @@ __global__ void __launch_bounds__(kHexBlock, kHexVjpBlocks) k_hex8_vjp(GaussBloc
     pdl_trigger();
     if (g >= last) return;
     int2 n = hex_edge_pair(b.conn, elem(g), p);
-    int32_t n0 = b.conn[8 * elem(g)];
     const double sig = (p == 1 || p == 2) ? -1.0 : 1.0;
     constexpr double s3 = kHexScale * kHexScale * kHexScale;
     for (; g < last; g += NW) {
         const int32_t e = elem(g);
+        const int32_t n0 = __shfl_sync(kFull, n.x, lane & ~3);
         HexRaw X, U, V;
         X.load<false>(X4, n0, n);
         double lam, mu;
@@ -2491,10 +2541,7 @@ __global__ void __launch_bounds__(kHexBlock, kHexVjpBlocks) k_hex8_vjp(GaussBloc
         pdl_wait();  // at once after the first round
         U.load<true>(U4, n0, n);
         V.load<true>(L4, n0, n);
-        if (g + NW < last) {
-            n = hex_edge_pair(b.conn, elem(g + NW), p);
-            n0 = b.conn[8 * elem(g + NW)];
-        }
+        if (g + NW < last) n = hex_edge_pair(b.conn, elem(g + NW), p);
         double J0[3], G0[3], W0[3];
         HexPair<double> v[3], J1[3], J2[3], G1[3], G2[3], W1[3], W2[3];
         X.rel<double>(v);
@@ -2712,6 +2759,16 @@ __global__ void __launch_bounds__(256) k_fbar_cell_vjp(CellBlockDev b, double* _
     store_theta(gmu, gk, s, -V * (ldm - 2.0 / 3.0 * ldl), -V * ldl, accumulate);
 }
 
+__device__ __forceinline__ void load_cell12(const double* p, double* g) {
+    const double2* q = reinterpret_cast<const double2*>(p);
+#pragma unroll
+    for (int k = 0; k < 6; ++k) {
+        const double2 v = __ldg(q + k);
+        g[2 * k] = v.x;
+        g[2 * k + 1] = v.y;
+    }
+}
+
 // VJP of the split-hex-grouped cells (FP64, one thread per patch): the cell VJP above
 // for the patch's six cells, summed per patch node.
 template <int MAT>
@@ -2730,7 +2787,7 @@ __global__ void __launch_bounds__(64) k_cell_hex6_vjp(CellBlockDev b, const doub
         const int64_t c = c0 + t;
         const int ln[4] = {0, kRing[t], kRing[t + 1], 3};
         double g[12];
-        load_cell12<double>(b.grads64 + 12 * c, g);
+        load_cell12(b.grads64 + 12 * c, g);
         double H[9], L[9];
 #pragma unroll
         for (int k = 0; k < 9; ++k) H[k] = L[k] = 0.0;
@@ -3926,6 +3983,13 @@ void launch_tet4_geometry(const int32_t* conn, int64_t num_elems, const double4*
     k_tet4_geometry<<<grid_for(num_elems, 256), 256, 0, s>>>(conn, num_elems, X4, geo32, geo64);
 }
 
+void launch_cell_units(const double* grads, const double* volumes, int64_t num_patches, float* unit32, double* unit64,
+                       cudaStream_t stream) {
+    if (num_patches <= 0) return;
+    k_cell_units<<<grid_for(20 * num_patches, 256), 256, 0, stream>>>(grads, volumes, 2 * num_patches,
+                                                                      reinterpret_cast<float4*>(unit32),
+                                                                      reinterpret_cast<double4*>(unit64));
+}
 void launch_hex6_patch_dx(const int32_t* patch_nodes, int64_t num_patches, const double4* X4, float* dx32,
                           double* dx64, cudaStream_t stream) {
     if (num_patches <= 0) return;

@@ -111,6 +111,11 @@ struct CellBlockDev {
     int64_t num_patches;
     const int32_t* patch_first;
     const int32_t* patch_nodes;
+    // Such cells' gradients and volumes by half patch, as k_cell_hex6_force's threads read them:
+    // unit 2q + r (cells 6q + 3r + k, k = 0, 1, 2) has vec4 number m at m * 2 num_patches + unit;
+    // numbers 3k .. 3k+2 are cell k's twelve gradient values, number 9 the three volumes.
+    const float* unit32;
+    const double* unit64;
     // F-bar (ComputeInternalForceSmoothedCell.h:354-413): the cells above are subcells,
     // grouped into num_groups cells by group_ptr; fbar is the per-subcell scratch
     // (kFbarStride values of the slot precision: H, J, then the stress). null: no F-bar.
@@ -193,6 +198,9 @@ void launch_gauss_vjp(const GaussBlockDev& b, const double4* X4, const double4* 
 // Lm: scratch of 9 doubles per cell for F-bar blocks (null otherwise). Returns the launch count.
 int launch_cell_vjp(const CellBlockDev& b, const double4* U4, const double4* L4, double* Lm, double4* slots,
                     double* gmu, double* gkappa, int accumulate, cudaStream_t s);
+// The half-patch tables of four-entry cells grouped as split hexes (see CellBlockDev::unit32).
+void launch_cell_units(const double* grads, const double* volumes, int64_t num_patches, float* unit32, double* unit64,
+                       cudaStream_t stream);
 void launch_hex6_patch_dx(const int32_t* patch_nodes, int64_t num_patches, const double4* X4, float* dx32,
                           double* dx64, cudaStream_t stream);
 void launch_gauss_volume_slots(const GaussBlockDev& b, double density, const double4* X4, double4* slots,

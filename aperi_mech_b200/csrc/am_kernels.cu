@@ -65,8 +65,7 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 
 // Loads of run-invariant data that a kernel reads once (connectivity, tables, plans): the
 // read-only path without an L1 line, which the nodal gathers beside them then keep. On B200,
-// us a step: smoothed cells of the h = 1/46 box mixed 33.2 -> 30.6, 128^3 Hex8 mixed 397 ->
-// 389, renumbered tets FP64 50.7 -> 49.1, 50 adjoint steps of 64^3 Hex8 15.1 -> 14.5 ms.
+// us a step: smoothed cells of the h = 1/46 box mixed 33.2 -> 30.6, renumbered tets FP64 50.7 -> 49.1, 50 adjoint steps of 64^3 Hex8 15.1 -> 14.5 ms.
 // Not for sectors that two loads share (patch nodes, reference differences): 30.6 -> 31.7 and,
 // split-hex tets mixed, 47.4 -> 47.6.
 __device__ __forceinline__ int32_t ld_once(const int32_t* p) {
@@ -915,15 +914,12 @@ __device__ __forceinline__ void hex_conn(const GaussBlockDev& b, int64_t e, int3
 // s_zeta, which H = G J^-1 does not see either and which leave one factor s_eta s_zeta on
 // det J and on the forces. The nodal sums run the same stages transposed.
 //
-// One thread per element held the 42 coefficients of X and u and 21 sums beside a Gauss
-// point's tensors: 246 registers and eight warps per SM in FP64, and 250 warps in all on
-// 8,000 elements. A quad's lane needs 128 (FP64) or 96 registers and a quarter of the
-// serial work. Measured on B200 (1965 MHz), one thread per element against this kernel:
-// a step of 20^3 linear elastic FP64 10.8 -> 7.7 us; 128^3 neo-Hookean with fields, per
-// launch, FP64 523 -> 459 us, mixed 320 -> 306 us. FP64: the FP64 pipe is 53% busy (its
-// floor is 290 us at 128^3), gather latency takes the rest; mixed: L1 wavefronts (gathers,
-// shuffles and slot stores) 60% and gather latency. The mixed path packs the lane's two
-// Gauss points into sm_100's two-wide FP32 operations.
+// FP64. One thread per element held the 42 coefficients of X and u and 21 sums beside a Gauss
+// point's tensors: 246 registers and eight warps per SM, and 250 warps in all on 8,000
+// elements. A quad's lane needs 128 registers and a quarter of the serial work. Measured on
+// B200 (1965 MHz), one thread per element against this kernel: a step of 20^3 linear elastic
+// 10.8 -> 7.7 us; 128^3 neo-Hookean with fields, per launch, 523 -> 459 us. The FP64 pipe is
+// 53% busy (its floor is 290 us at 128^3), gather latency takes the rest.
 // ---------------------------------------------------------------------------
 constexpr double kHexR = 0.26794919243112270647;   // (1 - c) / (1 + c) = 2 - sqrt 3
 constexpr double kHexScale = 0.31100423396407310780;  // (1 + c)^2 / 8: derivative = kHexScale x raw
@@ -933,10 +929,6 @@ template <typename T>
 struct HexPair {
     T a, b;  // at the xi = -1 and xi = +1 nodes (or Gauss points) of the lane
 };
-__device__ __forceinline__ HexPair<float> hp_fma(float k, const HexPair<float>& x, const HexPair<float>& y) {
-    const float2 v = vfma(make_float2(k, k), make_float2(x.a, x.b), make_float2(y.a, y.b));
-    return {v.x, v.y};
-}
 __device__ __forceinline__ HexPair<double> hp_fma(double k, const HexPair<double>& x, const HexPair<double>& y) {
     return {fma(k, x.a, y.a), fma(k, x.b, y.b)};
 }
@@ -949,10 +941,6 @@ template <typename T>
 __device__ __forceinline__ HexPair<T> hp_interp(const HexPair<T>& x) {
     const T r = T(kHexR);
     return {fma(r, x.b, x.a), fma(r, x.a, x.b)};
-}
-__device__ __forceinline__ HexPair<float> hp_scale(float k, const HexPair<float>& x) {
-    const float2 v = vmul(make_float2(k, k), make_float2(x.a, x.b));
-    return {v.x, v.y};
 }
 __device__ __forceinline__ HexPair<double> hp_scale(double k, const HexPair<double>& x) { return {k * x.a, k * x.b}; }
 
@@ -978,44 +966,44 @@ __device__ __forceinline__ HexPair<T> hex_transpose(T z, const HexPair<T>& q1, c
     return hp_fma(T(1), hp_xor(hp_fma(-r, w, v), 1), hp_fma(T(1), w, v));
 }
 
-// Q = adj(J) P^T at a Gauss point (two for float2) from J and the displacement gradient G
+// Q = adj(J) P^T at a Gauss point from J and the displacement gradient G
 // in the same raw units; sig = s_eta s_zeta. Returns whether det J and (neo-Hookean) det F
 // are positive.
-template <typename V, int MAT>
-__device__ __forceinline__ bool hex_gauss_q(const V* J, const V* G, double lam, double mu, double sig, V* Q) {
-    V A[9];
-    vadj3(J, A);
-    const V det = vfma(J[2], A[6], vfma(J[1], A[3], vmul(J[0], A[0])));
-    bool ok = all_positive(vmul(vset<V>(sig), det));
-    const V id = vrecip(det);
-    V H[9];
+template <int MAT>
+__device__ __forceinline__ bool hex_gauss_q(const double* J, const double* G, double lam, double mu, double sig, double* Q) {
+    double A[9];
+    adj3(J, A);
+    const double det = vfma(J[2], A[6], vfma(J[1], A[3], vmul(J[0], A[0])));
+    bool ok = sig * det > 0.0;
+    const double id = 1.0 / det;
+    double H[9];
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = 0; j < 3; ++j)
             H[i * 3 + j] = vmul(vfma(G[i * 3 + 2], A[6 + j], vfma(G[i * 3 + 1], A[3 + j], vmul(G[i * 3 + 0], A[j]))), id);
-    const V m = vset<V>(mu);
+    const double m = mu;
     if (MAT == kNeoHookean) {
         // Q = adj(J) P^T with P = tau F^-T and F = (J + G) J^-1 is adj(J + G) tau / det F
         // (the scale of J and G cancels): no F^-1 and no P.
-        V lln, iJ;
+        double lln, iJ;
         ok = nh_scalars(H, lam, lln, iJ) && ok;
-        const V sm = vmul(m, iJ), sl = vmul(lln, iJ);
-        V ts[9];
+        const double sm = vmul(m, iJ), sl = vmul(lln, iJ);
+        double ts[9];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int j = i; j < 3; ++j) {
-                V t = vadd(H[i * 3 + j], H[j * 3 + i]);
+                double t = vadd(H[i * 3 + j], H[j * 3 + i]);
 #pragma unroll
                 for (int k = 0; k < 3; ++k) t = vfma(H[i * 3 + k], H[j * 3 + k], t);
                 t = i == j ? vfma(sm, t, sl) : vmul(sm, t);
                 ts[i * 3 + j] = ts[j * 3 + i] = t;
             }
-        V Jc[9], Ac[9];
+        double Jc[9], Ac[9];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) Jc[k] = vadd(J[k], G[k]);
-        vadj3(Jc, Ac);
+        for (int k = 0; k < 9; ++k) Jc[k] = J[k] + G[k];
+        adj3(Jc, Ac);
 #pragma unroll
         for (int k = 0; k < 3; ++k)
 #pragma unroll
@@ -1023,31 +1011,31 @@ __device__ __forceinline__ bool hex_gauss_q(const V* J, const V* G, double lam, 
                 Q[k * 3 + i] = vfma(Ac[k * 3 + 2], ts[6 + i], vfma(Ac[k * 3 + 1], ts[3 + i], vmul(Ac[k * 3 + 0], ts[i])));
         return ok;
     }
-    V P[9];
-    const V l = vset<V>(lam);
+    double P[9];
+    const double l = lam;
     if (MAT == kLinearElastic) {
-        const V tr = vmul(l, vadd(vadd(H[0], H[4]), H[8]));
+        const double tr = vmul(l, vadd(vadd(H[0], H[4]), H[8]));
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int j = i; j < 3; ++j) {
-                const V e = vadd(H[i * 3 + j], H[j * 3 + i]);
+                const double e = vadd(H[i * 3 + j], H[j * 3 + i]);
                 P[i * 3 + j] = P[j * 3 + i] = i == j ? vfma(m, e, tr) : vmul(m, e);
             }
     } else {
         // 2E = H + H^T + H^T H, S = lambda/2 tr(2E) I + mu 2E, P = S + H S
-        V E[9];
+        double E[9];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int j = i; j < 3; ++j) {
-                V e = vadd(H[i * 3 + j], H[j * 3 + i]);
+                double e = vadd(H[i * 3 + j], H[j * 3 + i]);
 #pragma unroll
                 for (int k = 0; k < 3; ++k) e = vfma(H[k * 3 + i], H[k * 3 + j], e);
                 E[i * 3 + j] = E[j * 3 + i] = e;
             }
-        const V tr = vmul(vset<V>(0.5 * lam), vadd(vadd(E[0], E[4]), E[8]));
-        V S[9];
+        const double tr = vmul(0.5 * lam, vadd(vadd(E[0], E[4]), E[8]));
+        double S[9];
 #pragma unroll
         for (int k = 0; k < 9; ++k) S[k] = k % 4 == 0 ? vfma(m, E[k], tr) : vmul(m, E[k]);
 #pragma unroll
@@ -1089,21 +1077,19 @@ struct HexRaw {
     }
 };
 
-// Sixteen (FP64, 128 registers) or twenty (FP32) warps per SM.
-template <typename T>
-constexpr int hex_min_blocks() { return sizeof(T) == 4 ? 5 : 4; }
+constexpr int kHexBlocks = 4;  // sixteen warps per SM, 128 registers
 
 // Rounds of eight elements a warp runs: as many as keep three waves of 148 x 16 warps, at
 // most eight. From the second round on a warp has its connectivity at hand. Measured on
-// B200 at 128^3, neo-Hookean with fields (us per launch, 1 / 2 / 4 / 8 rounds): FP64 497 /
-// 480 / 476 / 459, mixed 344 / 321 / 311 / 306. Fewer waves leave SMs empty: 20^3 linear elastic FP64 took
+// B200 at 128^3, neo-Hookean with fields (us per launch, 1 / 2 / 4 / 8 rounds): 497 / 480 /
+// 476 / 459. Fewer waves leave SMs empty: 20^3 linear elastic FP64 took
 // 7.7 us a step with one round, 8.1 with two and 11.7 with four.
 inline int32_t hex_rounds(int64_t groups) { return static_cast<int32_t>(std::clamp<int64_t>(groups / (3 * 148 * 16), 1, 8)); }
 
-template <typename T, int MAT>
-__global__ void __launch_bounds__(kHexBlock, hex_min_blocks<T>()) k_hex8_force(GaussBlockDev b, const double4* __restrict__ X4,
+template <int MAT>
+__global__ void __launch_bounds__(kHexBlock, kHexBlocks) k_hex8_force(GaussBlockDev b, const double4* __restrict__ X4,
                                                           const double4* __restrict__ U4,
-                                                          vec4_t<T>* __restrict__ slots, int* status, int32_t rounds) {
+                                                          double4* __restrict__ slots, int* status, int32_t rounds) {
     constexpr int W = kHexBlock / 32;
     const int lane = static_cast<int>(threadIdx.x & 31), p = lane & 3;
     const int32_t E = static_cast<int32_t>(b.num_elems);
@@ -1129,76 +1115,155 @@ __global__ void __launch_bounds__(kHexBlock, hex_min_blocks<T>()) k_hex8_force(G
         U.load<true>(U4, n0, n);
         // the next group's connectivity travels while this one is computed
         if (g + W < last) n = hex_edge_pair(b.conn, elem(g + W), p);
-        HexPair<T> x[3], u[3];
-        X.rel<T>(x);
-        U.rel<T>(u);
-        T J0[3], G0[3];
-        HexPair<T> J1[3], J2[3], G1[3], G2[3];
+        HexPair<double> x[3], u[3];
+        X.rel<double>(x);
+        U.rel<double>(u);
+        double J0[3], G0[3];
+        HexPair<double> J1[3], J2[3], G1[3], G2[3];
 #pragma unroll
         for (int i = 0; i < 3; ++i) hex_derivatives(x[i], J0[i], J1[i], J2[i]);
 #pragma unroll
         for (int i = 0; i < 3; ++i) hex_derivatives(u[i], G0[i], G1[i], G2[i]);
-        T z[3];
-        HexPair<T> q1[3], q2[3];
-        bool ok;
-        if constexpr (sizeof(T) == 4) {
-            float2 J[9], G[9], Q[9];
+        double z[3];
+        HexPair<double> q1[3], q2[3];
+        bool ok = true;
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            double J[9], G[9], Q[9];
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
-                J[3 * i] = make_float2(J0[i], J0[i]);
-                J[3 * i + 1] = make_float2(J1[i].a, J1[i].b);
-                J[3 * i + 2] = make_float2(J2[i].a, J2[i].b);
-                G[3 * i] = make_float2(G0[i], G0[i]);
-                G[3 * i + 1] = make_float2(G1[i].a, G1[i].b);
-                G[3 * i + 2] = make_float2(G2[i].a, G2[i].b);
+                J[3 * i] = J0[i];
+                J[3 * i + 1] = h ? J1[i].b : J1[i].a;
+                J[3 * i + 2] = h ? J2[i].b : J2[i].a;
+                G[3 * i] = G0[i];
+                G[3 * i + 1] = h ? G1[i].b : G1[i].a;
+                G[3 * i + 2] = h ? G2[i].b : G2[i].a;
             }
-            ok = hex_gauss_q<float2, MAT>(J, G, lam, mu, sig, Q);
+            ok = hex_gauss_q<MAT>(J, G, lam, mu, sig, Q) && ok;
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
-                z[i] = Q[i].x + Q[i].y;
-                q1[i] = {Q[3 + i].x, Q[3 + i].y};
-                q2[i] = {Q[6 + i].x, Q[6 + i].y};
-            }
-        } else {
-            ok = true;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                double J[9], G[9], Q[9];
-#pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    J[3 * i] = J0[i];
-                    J[3 * i + 1] = h ? J1[i].b : J1[i].a;
-                    J[3 * i + 2] = h ? J2[i].b : J2[i].a;
-                    G[3 * i] = G0[i];
-                    G[3 * i + 1] = h ? G1[i].b : G1[i].a;
-                    G[3 * i + 2] = h ? G2[i].b : G2[i].a;
-                }
-                ok = hex_gauss_q<double, MAT>(J, G, lam, mu, sig, Q) && ok;
-#pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    if (h == 0) {
-                        z[i] = Q[i];
-                        q1[i].a = Q[3 + i];
-                        q2[i].a = Q[6 + i];
-                    } else {
-                        z[i] += Q[i];
-                        q1[i].b = Q[3 + i];
-                        q2[i].b = Q[6 + i];
-                    }
+                if (h == 0) {
+                    z[i] = Q[i];
+                    q1[i].a = Q[3 + i];
+                    q2[i].a = Q[6 + i];
+                } else {
+                    z[i] += Q[i];
+                    q1[i].b = Q[3 + i];
+                    q2[i].b = Q[6 + i];
                 }
             }
         }
         const bool valid = 8 * g + (lane >> 2) < E;
         if (!ok && valid) flag(status, AM_ENONPOS_J, e);
-        const T s = T(-sig * kHexScale * kHexScale * kHexScale);
-        HexPair<T> f[3];
+        HexPair<double> f[3];
 #pragma unroll
-        for (int i = 0; i < 3; ++i) f[i] = hp_scale(s, hex_transpose(z[i], q1[i], q2[i]));
+        for (int i = 0; i < 3; ++i)
+            f[i] = hp_scale(-sig * kHexScale * kHexScale * kHexScale, hex_transpose(z[i], q1[i], q2[i]));
         if (valid) {
             slots[pos.x] = make4(f[0].a, f[1].a, f[2].a);
             slots[pos.y] = make4(f[0].b, f[1].b, f[2].b);
         }
     }
+}
+
+// The mixed path: one thread per element in the monomial basis (see hex_butterfly), 128
+// registers and four 128-thread blocks per SM. The quads above, with a lane's two Gauss points
+// in sm_100's two-wide FP32 operations, ran 128^3 in 306 against 320 us but rounded the
+// Gauss-point weights of every element alike: after 1000 steps of that mesh's noise problem
+// the displacement was 6.5e-6 to 1.4e-5 from FP64's, against 1.4e-6 here.
+template <int MAT>
+__global__ void __launch_bounds__(128, 4) k_hex8_force_mixed(GaussBlockDev b, const double4* __restrict__ X4,
+                                                         const double4* __restrict__ U4,
+                                                         float4* __restrict__ slots, int* status) {
+    using T = float;
+    const int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (e >= b.num_elems) return;
+    int32_t nd[8];
+    hex_conn(b, e, nd);
+    T X[3][8], U[3][8];
+    hex_load_rel(X4, nd, X);
+    pdl_trigger();
+    pdl_wait();
+    hex_load_rel<T, true>(U4, nd, U);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        hex_butterfly(X[i]);
+        hex_butterfly(U[i]);
+        hex_scale_coeffs(X[i]);
+        hex_scale_coeffs(U[i]);
+    }
+    double lam, mu;
+    element_lame(b, e, lam, mu);
+    T R[3][8];
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) R[i][k] = T(0);
+    bool bad = false;
+#pragma unroll 2
+    for (int g = 0; g < 8; ++g) {
+        T J[9], G[9], A[9];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                J[i * 3 + j] = hex_dxi(X[i], j, g);
+                G[i * 3 + j] = hex_dxi(U[i], j, g);
+            }
+        adj3(J, A);
+        const T det = J[0] * A[0] + J[1] * A[3] + J[2] * A[6];
+        bad |= !(det > T(0));
+        const T id = recip(det);
+        T H[9], P[9];
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j)
+                H[i * 3 + j] = (G[i * 3 + 0] * A[0 * 3 + j] + G[i * 3 + 1] * A[1 * 3 + j] + G[i * 3 + 2] * A[2 * 3 + j]) * id;
+        T Q[9];
+        if (MAT == kNeoHookean) {
+            // Q = adj(J) P^T with P = tau F^-T and F = (J + G) J^-1 is adj(J + G) tau / det F
+            // (the 8x scale of J and G cancels): no F^-1 and no P.
+            T tau[9];
+            const double Jf = nh_kirchhoff<T>(T(lam), T(mu), H, tau);
+            bad |= !(Jf > 0.0);
+            T Jc[9], Ac[9];
+#pragma unroll
+            for (int k = 0; k < 9; ++k) Jc[k] = J[k] + G[k];
+            adj3(Jc, Ac);
+            const T sc = sizeof(T) == 4 ? T(__frcp_rn(static_cast<float>(Jf))) : T(1.0 / Jf);
+            T ts[9];
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+#pragma unroll
+                for (int j = i; j < 3; ++j) ts[i * 3 + j] = ts[j * 3 + i] = sc * tau[i * 3 + j];
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+                    Q[k * 3 + i] = Ac[k * 3 + 0] * ts[0 * 3 + i] + Ac[k * 3 + 1] * ts[1 * 3 + i] + Ac[k * 3 + 2] * ts[2 * 3 + i];
+        } else {
+            stress<T>(MAT, T(lam), T(mu), H, P);
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+#pragma unroll
+                for (int i = 0; i < 3; ++i)
+                    Q[k * 3 + i] = A[k * 3 + 0] * P[i * 3 + 0] + A[k * 3 + 1] * P[i * 3 + 1] + A[k * 3 + 2] * P[i * 3 + 2];
+        }
+        hex_accumulate_r(R, Q, g);
+    }
+    if (bad) flag(status, AM_ENONPOS_J, e);
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        R[i][0] = T(0);
+        hex_scale_coeffs(R[i]);
+        hex_butterfly_t(R[i]);
+    }
+    const T s = T(-1.0 / 512.0);
+    const int4 p0 = reinterpret_cast<const int4*>(b.slot_pos)[2 * e], p1 = reinterpret_cast<const int4*>(b.slot_pos)[2 * e + 1];
+    const int32_t pos[8] = {p0.x, p0.y, p0.z, p0.w, p1.x, p1.y, p1.z, p1.w};
+#pragma unroll
+    for (int q = 0; q < 8; ++q) slots[pos[hex_node_of_corner(q)]] = make4(s * R[0][q], s * R[1][q], s * R[2][q]);
 }
 
 // ---------------------------------------------------------------------------
@@ -3134,10 +3199,33 @@ __global__ void __launch_bounds__(256) k_prologue(NodeDev nd, const StepParams* 
     if (u_copy) u_copy[i] = u;
 }
 
+// The step's scalars that every node takes from the step table, loaded by the node kernel
+// before its wait for the element kernels (the table is written before the run's first kernel,
+// or before the graph): after it they were one more dependent load on every node's chain. On
+// B200, us a step: 20^3 Hex8 FP64 (launch-bound) 7.46 -> 7.11, split-hex tets FP64 39.8 -> 39.3,
+// smoothed cells mixed 30.6 -> 30.0. The coupling's columns load them late: eight more
+// registers there cost a block per SM (43.5 -> 47.2).
+struct StepScalars {
+    double half, half_next, dt_next;
+    uint32_t aact, vact_next;
+};
+__device__ __forceinline__ StepScalars step_scalars(const StepParams* __restrict__ table, int64_t step, int advance) {
+    const StepParams& P = table[step];
+    StepScalars s{P.half, 0.0, 0.0, P.aact, 0u};
+    if (advance) {
+        const StepParams& Q = table[step + 1];
+        s.half_next = Q.half;
+        s.dt_next = Q.dt;
+        s.vact_next = Q.vact;
+    }
+    return s;
+}
+
 // The central-difference update of node i from its force (mass m, BC word w, half-step
 // velocity vh, displacement u0, which is read only when advance is set).
 __device__ __forceinline__ void node_update(const NodeDev& nd, int64_t i, double fx, double fy, double fz, double m, uint32_t w,
-                                            const double4& vh, const double4& u0, const StepParams* __restrict__ table,
+                                            const double4& vh, const double4& u0, const StepScalars& sc,
+                                            const StepParams* __restrict__ table,
                                             int64_t step, int advance, double4* __restrict__ U4, double4* __restrict__ V4,
                                             double4* __restrict__ A4, double4* __restrict__ u_copy, int* status, int rebase) {
     if (nd.has_g) {
@@ -3148,18 +3236,18 @@ __device__ __forceinline__ void node_update(const NodeDev& nd, int64_t i, double
     // a^{n+1} = f / m (ExplicitTimeIntegrator.h:247-283), then the acceleration BC at t^{n+1}.
     double ax = fx / m, ay = fy / m, az = fz / m;
     const StepParams& P = table[step];
-    if (w) apply_bc(w, P.aact, P.ascale, nd.bcvalues, ax, ay, az);
+    if (w) apply_bc(w, sc.aact, P.ascale, nd.bcvalues, ax, ay, az);
     if (!isfinite(ax) || !isfinite(ay) || !isfinite(az)) flag(status, AM_ENAN, i);
     // v^{n+1} = v^{n+1/2} + dt/2 a^{n+1} (:329-364)
-    const double vx = vh.x + P.half * ax, vy = vh.y + P.half * ay, vz = vh.z + P.half * az;
+    const double vx = vh.x + sc.half * ax, vy = vh.y + sc.half * ay, vz = vh.z + sc.half * az;
     if (advance) {
         // Next step: v^{n+3/2} = v^{n+1} + dt'/2 a^{n+1} (:286-326), velocity BC at t_mid',
         // u^{n+2} = u^{n+1} + dt' v^{n+3/2} (:97-134).
         const StepParams& Q = table[step + 1];
-        double wx = vx + Q.half * ax, wy = vy + Q.half * ay, wz = vz + Q.half * az;
-        if (w) apply_bc(w, Q.vact, Q.vscale, nd.bcvalues, wx, wy, wz);
+        double wx = vx + sc.half_next * ax, wy = vy + sc.half_next * ay, wz = vz + sc.half_next * az;
+        if (w) apply_bc(w, sc.vact_next, Q.vscale, nd.bcvalues, wx, wy, wz);
         double4 u = u0;
-        displace(nd, i, rebase, Q.dt, wx, wy, wz, u);
+        displace(nd, i, rebase, sc.dt_next, wx, wy, wz, u);
         st4(U4 + i, u);
         st4(V4 + i, make_double4(wx, wy, wz, 0.0));
         if (u_copy) st4(u_copy + i, u);
@@ -3169,8 +3257,10 @@ __device__ __forceinline__ void node_update(const NodeDev& nd, int64_t i, double
     }
 }
 
+// FP32 slots in batches of eight are held to the 72 registers of seven blocks per SM (75
+// without: 47.2 -> 48.1 us a step on the split-hex 70^3 mesh).
 template <typename S, int BATCH, int LPN>
-__global__ void __launch_bounds__(kNodeBlock) k_node_step(NodeDev nd, const vec4_t<S>* __restrict__ slots,
+__global__ void __launch_bounds__(kNodeBlock, sizeof(S) == 4 && BATCH == 8 ? 7 : 0) k_node_step(NodeDev nd, const vec4_t<S>* __restrict__ slots,
                                                            const StepParams* __restrict__ table, int64_t step,
                                                            int advance, double4* __restrict__ U4,
                                                            double4* __restrict__ V4, double4* __restrict__ A4,
@@ -3191,6 +3281,7 @@ __global__ void __launch_bounds__(kNodeBlock) k_node_step(NodeDev nd, const vec4
     const double m = nd.mass[j];
     const uint32_t w = nd.bcword[j];
     const NodeSlots q = node_slots(nd, i, own);
+    const StepScalars sc = step_scalars(table, step, advance);
     pdl_trigger();
     pdl_wait();
     const double4 vh = ld_dep(V4 + j);
@@ -3198,7 +3289,7 @@ __global__ void __launch_bounds__(kNodeBlock) k_node_step(NodeDev nd, const vec4
     double fx, fy, fz;
     gather<S, BATCH, LPN>(nd, slots, i, own, q, fx, fy, fz);
     if (!own || threadIdx.x % LPN != 0) return;
-    node_update(nd, i, fx, fy, fz, m, w, vh, u0, table, step, advance, U4, V4, A4, u_copy, status, rebase);
+    node_update(nd, i, fx, fy, fz, m, w, vh, u0, sc, table, step, advance, U4, V4, A4, u_copy, status, rebase);
 }
 
 // Reverse of the acceleration step: lam = Ma (abar + h vbar) / m, the cotangent
@@ -3500,7 +3591,7 @@ __global__ void __launch_bounds__(kOctetBlock) k_rk_octets(int64_t count, int64_
     }
     if (!mine) return;
     if (STEP) {
-        node_update(a.nd, i, x, y, z, m, bc, vh, u0, a.table, a.step, a.advance, a.U4, a.V4, a.A4, a.u_copy, a.status, 0);
+        node_update(a.nd, i, x, y, z, m, bc, vh, u0, step_scalars(a.table, a.step, a.advance), a.table, a.step, a.advance, a.U4, a.V4, a.A4, a.u_copy, a.status, 0);
     } else if (out4 != nullptr) {
         st4(out4 + i, row_ptr[i + 1] != row_ptr[i] ? make_double4(x, y, z, 0.0)
                       : i < num_nodes              ? ld_dep(in + i)
@@ -3743,13 +3834,12 @@ void launch_gauss_force(const GaussBlockDev& b, int mixed, const double4* X4, co
             AM_DISPATCH_MAT(b.material, (k_tet4_force<double, M><<<grid, 256, 0, s>>>(b, X4, U4, static_cast<double4*>(slots), status)));
         }
     } else {
-        const int64_t groups = (b.num_elems + 7) / 8;
-        const int32_t rounds = hex_rounds(groups);
-        const unsigned grid = grid_for(groups, rounds * (kHexBlock / 32));
         if (mixed) {
-            AM_DISPATCH_MAT(b.material, (launch_pdl(k_hex8_force<float, M>, grid, kHexBlock, s, b, X4, U4, static_cast<float4*>(slots), status, rounds)));
+            AM_DISPATCH_MAT(b.material, (launch_pdl(k_hex8_force_mixed<M>, grid_for(b.num_elems, 128), 128, s, b, X4, U4, static_cast<float4*>(slots), status)));
         } else {
-            AM_DISPATCH_MAT(b.material, (launch_pdl(k_hex8_force<double, M>, grid, kHexBlock, s, b, X4, U4, static_cast<double4*>(slots), status, rounds)));
+            const int64_t groups = (b.num_elems + 7) / 8;
+            const int32_t rounds = hex_rounds(groups);
+            AM_DISPATCH_MAT(b.material, (launch_pdl(k_hex8_force<M>, grid_for(groups, rounds * (kHexBlock / 32)), kHexBlock, s, b, X4, U4, static_cast<double4*>(slots), status, rounds)));
         }
     }
 }

@@ -157,78 +157,19 @@ __device__ __forceinline__ double stress(int32_t mat, T lambda, T mu, const T* H
     return 1.0;
 }
 
-// ---------------------------------------------------------------------------
-// Two Gauss points side by side: a value V is a float2 (one FP32 value per point, in
-// sm_100's packed add / multiply / fma, half the issue slots of scalar FP32) or a plain
-// double (one point at a time). v* write every fused operation out, as the packed
-// intrinsics are not contracted by the compiler.
-// ---------------------------------------------------------------------------
-__device__ __forceinline__ float2 vadd(float2 x, float2 y) { return __fadd2_rn(x, y); }
-__device__ __forceinline__ float2 vmul(float2 x, float2 y) { return __fmul2_rn(x, y); }
-__device__ __forceinline__ float2 vfma(float2 x, float2 y, float2 z) { return __ffma2_rn(x, y, z); }
-__device__ __forceinline__ float2 vneg(float2 x) { return __fmul2_rn(x, make_float2(-1.f, -1.f)); }
-__device__ __forceinline__ float2 vsub(float2 x, float2 y) { return __ffma2_rn(y, make_float2(-1.f, -1.f), x); }
+// Fused operations written out (Hex8 quads), so that their order does not depend on the
+// compiler's contraction.
 __device__ __forceinline__ double vadd(double x, double y) { return x + y; }
 __device__ __forceinline__ double vmul(double x, double y) { return x * y; }
 __device__ __forceinline__ double vfma(double x, double y, double z) { return fma(x, y, z); }
-__device__ __forceinline__ double vneg(double x) { return -x; }
-__device__ __forceinline__ double vsub(double x, double y) { return x - y; }
-// The same scalar at both points.
-template <typename V>
-__device__ __forceinline__ V vset(double x);
-template <>
-__device__ __forceinline__ float2 vset<float2>(double x) { return make_float2(static_cast<float>(x), static_cast<float>(x)); }
-template <>
-__device__ __forceinline__ double vset<double>(double x) { return x; }
-__device__ __forceinline__ float2 vrecip(float2 x) { return make_float2(recip(x.x), recip(x.y)); }
-__device__ __forceinline__ double vrecip(double x) { return 1.0 / x; }
-__device__ __forceinline__ bool all_positive(float2 x) { return x.x > 0.f && x.y > 0.f; }
-__device__ __forceinline__ bool all_positive(double x) { return x > 0.0; }
 
-// adj3 with the six negated entries its products share (packed operands carry no sign).
-template <typename V>
-__device__ __forceinline__ void vadj3(const V* m, V* r) {
-    V n[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) n[k] = vneg(m[k]);
-    r[0] = vfma(m[4], m[8], vmul(n[5], m[7]));
-    r[1] = vfma(m[2], m[7], vmul(n[1], m[8]));
-    r[2] = vfma(m[1], m[5], vmul(n[2], m[4]));
-    r[3] = vfma(m[5], m[6], vmul(n[3], m[8]));
-    r[4] = vfma(m[0], m[8], vmul(n[2], m[6]));
-    r[5] = vfma(m[2], m[3], vmul(n[0], m[5]));
-    r[6] = vfma(m[3], m[7], vmul(n[4], m[6]));
-    r[7] = vfma(m[1], m[6], vmul(n[0], m[7]));
-    r[8] = vfma(m[0], m[4], vmul(n[1], m[3]));
-}
-
-// Neo-Hookean log J and 1 / J (the two scalars its stress needs), FP64 as in nh_kirchhoff;
-// returns whether every J is positive.
+// Neo-Hookean log J and 1 / J (the two scalars its stress needs) as in nh_kirchhoff; returns
+// whether J is positive.
 __device__ __forceinline__ bool nh_scalars(const double* H, double lambda, double& lam_lnJ, double& iJ) {
     const double Jm1 = det_ap_im1(H), J = 1.0 + Jm1;
     lam_lnJ = lambda * log1p_nh(Jm1);
     iJ = 1.0 / J;
     return J > 0.0;
-}
-__device__ __forceinline__ bool nh_scalars(const float2* H, double lambda, float2& lam_lnJ, float2& iJ) {
-    bool ok = true;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        float Hs[9];
-#pragma unroll
-        for (int k = 0; k < 9; ++k) Hs[k] = h ? H[k].y : H[k].x;
-        const double Jm1 = det_ap_im1(Hs), J = 1.0 + Jm1;
-        const float l = static_cast<float>(lambda * log1p_nh(Jm1)), i = __frcp_rn(static_cast<float>(J));
-        if (h) {
-            lam_lnJ.y = l;
-            iJ.y = i;
-        } else {
-            lam_lnJ.x = l;
-            iJ.x = i;
-        }
-        ok = ok && J > 0.0;
-    }
-    return ok;
 }
 
 // Directional derivative dP[L] at H (equal to the vector-Jacobian product since

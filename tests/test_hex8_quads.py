@@ -1,4 +1,4 @@
-"""The four-lanes-per-element Hex8 force kernel where its grouping can go wrong: element
+"""The four-lanes-per-element Hex8 force kernel (FP64) where its grouping can go wrong: element
 counts around the eight elements of a warp and the 32 of a block, and blocks of several
 rounds (two from 2 x 3 x 148 x 16 x 8 elements on), with a last round that is not full.
 

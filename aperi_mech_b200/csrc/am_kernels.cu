@@ -65,7 +65,8 @@ __device__ __forceinline__ void prefetch_l2(const void* p) { asm volatile("prefe
 
 // Loads of run-invariant data that a kernel reads once (connectivity, tables, plans): the
 // read-only path without an L1 line, which the nodal gathers beside them then keep. On B200,
-// us a step: smoothed cells of the h = 1/46 box mixed 33.2 -> 30.6, renumbered tets FP64 50.7 -> 49.1, 50 adjoint steps of 64^3 Hex8 15.1 -> 14.5 ms.
+// us a step: smoothed cells of the h = 1/46 box mixed 33.2 -> 30.6, renumbered tets
+// FP64 50.7 -> 49.1, 50 adjoint steps of 64^3 Hex8 15.1 -> 14.5 ms.
 // Not for sectors that two loads share (patch nodes, reference differences): 30.6 -> 31.7 and,
 // split-hex tets mixed, 47.4 -> 47.6.
 __device__ __forceinline__ int32_t ld_once(const int32_t* p) {

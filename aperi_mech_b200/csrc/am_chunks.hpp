@@ -1,4 +1,5 @@
-// am_chunks.hpp -- warp-chunk plans of one-thread-per-element blocks (host code).
+// am_chunks.hpp -- warp-chunk plans of one-thread-per-element blocks, and where the blocks'
+// logical slots begin (host code).
 //
 // The force kernels of such blocks sum, per warp, the nodal forces of the warp's 32 units
 // (elements, or split-hex half patches) on each node they share, and write one slot per
@@ -72,6 +73,16 @@ inline bool build_warp_chunks(const int32_t* conn, int64_t E, int nn, WarpChunks
         t.ptr[c + 1] = t.ptr[c] + nd;
     }
     return true;
+}
+
+// First logical slot of each block from the blocks' logical slot counts, and behind them the
+// size of the slot-position array. Kernels read a block's positions two and four at a time, so
+// every block begins at a multiple of four whatever the blocks before it hold (a warp-chunked,
+// per-entry or cell-stress block may hold an odd number); positions in the gaps stay unused.
+inline std::vector<int64_t> slot_bases(const std::vector<int64_t>& counts) {
+    std::vector<int64_t> base(counts.size() + 1, 0);
+    for (size_t k = 0; k < counts.size(); ++k) base[k + 1] = (base[k] + counts[k] + 3) / 4 * 4;
+    return base;
 }
 
 }  // namespace am

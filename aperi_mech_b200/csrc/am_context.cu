@@ -215,7 +215,7 @@ struct Block {
     double lambda = 0, mu = 0, density = 0;
     int64_t num_elems = 0;
     int64_t num_entries = 0;  // slots of this block
-    int64_t slot_base = 0;
+    int64_t slot_base = 0;    // first logical slot, a multiple of four (am_finalize)
     int64_t slot_count = -1;  // logical slots when they differ from num_entries (patched cells)
     int32_t* conn = nullptr;
     double* mu_field = nullptr;
@@ -1640,7 +1640,6 @@ int am_add_block(am_ctx* ctx, const am_block_desc* d, int32_t* block_id) {
         b.mu = d->mu;
         b.density = d->density;
         b.num_elems = d->num_elems;
-        b.slot_base = ctx->num_slots;
         const int64_t E = d->num_elems;
         try {
             if (d->kind == AM_SMOOTHED_CELLS) {
@@ -1960,7 +1959,7 @@ int am_finalize(am_ctx* ctx) {
         // Generic cell blocks (without F-bar groups, or with groups of at most 32 subcells)
         // take the cell-stress form: one logical slot per node they touch instead of one per
         // entry.
-        int64_t base = 0;
+        std::vector<int64_t> counts;
         for (auto& b : ctx->blocks) {
             if (!b.host_grads.empty() && b.patched == 0 && (!b.group_ptr || b.cells().fused)) {
                 std::memcpy(b.unroll, ctx->cell_unroll, sizeof b.unroll);
@@ -1969,10 +1968,11 @@ int am_finalize(am_ctx* ctx) {
             std::vector<double>().swap(b.host_grads);
             std::vector<int32_t>().swap(b.host_cell_ptr);
             std::vector<int64_t>().swap(b.host_group_ptr);
-            b.slot_base = base;
-            base += static_cast<int64_t>(b.host_nodes.size());
+            counts.push_back(static_cast<int64_t>(b.host_nodes.size()));
         }
-        ctx->num_slots = base;
+        const std::vector<int64_t> base = am::slot_bases(counts);
+        for (size_t k = 0; k < ctx->blocks.size(); ++k) ctx->blocks[k].slot_base = base[k];
+        ctx->num_slots = base.back();
         const int64_t S = ctx->num_slots;
         // Node-major slot layout: node (or point) i owns positions [ptr[i], ptr[i+1]); within
         // a node the positions follow ascending logical slot (block order, then element order).

@@ -41,7 +41,7 @@ def _first_block(kind, coords, conn, mat):
         n = int(kind[4:])
         return Part("tet4", mat, conn=tets[:n])
     rng = np.random.default_rng(11)
-    sizes = (3, 4, 6) if kind == "entries" else (9, 11)  # one slot per entry / per touched node
+    sizes = (3, 4, 6) if kind == "entries" else (9, 12)  # one slot per entry / per touched node
     nodes = [rng.choice(coords.shape[0], size=s, replace=False) for s in sizes]
     grads = [rng.uniform(-1.0, 1.0, (s, 3)) for s in sizes]
     grads = [g - g.mean(axis=0) for g in grads]  # a constant field has no gradient

@@ -2498,10 +2498,14 @@ __global__ void __launch_bounds__(256) k_tet4_patch_vjp(GaussBlockDev b, const d
 // L = W J^-1 (J, G, W in the raw units of hex_derivatives, sig as in hex_gauss_q), and the
 // sensitivities L : dP/dlambda and L : dP/dmu at fixed H.
 // Neo-Hookean: dP^T = mu L^T + a F^-1 L F^-1 + lambda tr(F^-1 L) F^-1, a = mu - lambda log J.
-// With Jc = J + G (F = Jc J^-1) and M = J^-1 J^-T neither H, L nor F^-1 is formed:
-//   Q = det J (mu (W M)^T + a Jc^-1 W Jc^-1 + lambda tr(Jc^-1 W) Jc^-1),
-//   tr(F^-1 L) = tr(Jc^-1 W),  L : F = (W M) : Jc,
-//   J - 1 = (adj(J) : G^T + adj(G) : J^T + det G) / det J.
+// With Jc = J + G (F = Jc J^-1) F^-1 is not formed:
+//   Q = mu adj(J) L^T + det J (a Jc^-1 W Jc^-1 + lambda tr(Jc^-1 W) Jc^-1),
+//   tr(F^-1 L) = tr(W Jc^-1),  L : (F - F^-T) = (F F^T - I) : (W Jc^-1),
+// the last from H + H^T + H H^T, which is of the strain's order before the contraction, so that
+// nothing of order one cancels and no product has the condition of J twice.
+// Error of L : dP/dmu over the strain (J = R1 diag(1, 1, 1/k) R2, FP64 against long double):
+// k = 1: 1e-14, 100: 2e-13, 1000: 2e-12, at strains 1e-2 and 1e-4; L : (F - F^-T) entry by
+// entry 1e-11 at 1e-4, (W J^-1 J^-T) : Jc - tr 3e-8 at k = 100.
 template <int MAT>
 __device__ __forceinline__ double hex_gauss_vjp(const double* J, const double* G, const double* W, double lam, double mu,
                                                 double* Q, double& l_dlam, double& l_dmu) {
@@ -2509,62 +2513,54 @@ __device__ __forceinline__ double hex_gauss_vjp(const double* J, const double* G
     adj3(J, A);
     const double det = J[0] * A[0] + J[1] * A[3] + J[2] * A[6];
     const double id = 1.0 / det;
-    if (MAT == kNeoHookean) {
-        double B[9], Jc[9];
-        adj3(G, B);
-        double num = G[0] * B[0] + G[1] * B[3] + G[2] * B[6];
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-            for (int j = 0; j < 3; ++j) num += A[i * 3 + j] * G[j * 3 + i] + B[i * 3 + j] * J[j * 3 + i];
-        const double lnJ = log1p_nh(num * id);
-#pragma unroll
-        for (int k = 0; k < 9; ++k) Jc[k] = J[k] + G[k];
-        adj3(Jc, B);
-        const double ic = 1.0 / (det + num);
-        double C[9], N[9], S[6];
-#pragma unroll
-        for (int i = 0; i < 3; ++i)
-#pragma unroll
-            for (int j = 0; j < 3; ++j) C[i * 3 + j] = B[i * 3 + 0] * W[0 + j] + B[i * 3 + 1] * W[3 + j] + B[i * 3 + 2] * W[6 + j];
-        const double tr = (C[0] + C[4] + C[8]) * ic;
-        // S = adj(J) adj(J)^T (upper triangle), N = W M = W S / det^2
-        S[0] = A[0] * A[0] + A[1] * A[1] + A[2] * A[2];
-        S[1] = A[0] * A[3] + A[1] * A[4] + A[2] * A[5];
-        S[2] = A[0] * A[6] + A[1] * A[7] + A[2] * A[8];
-        S[3] = A[3] * A[3] + A[4] * A[4] + A[5] * A[5];
-        S[4] = A[3] * A[6] + A[4] * A[7] + A[5] * A[8];
-        S[5] = A[6] * A[6] + A[7] * A[7] + A[8] * A[8];
-        double lf = 0.0;
-#pragma unroll
-        for (int i = 0; i < 3; ++i) {
-            const double w0 = W[i * 3], w1 = W[i * 3 + 1], w2 = W[i * 3 + 2];
-            N[i * 3 + 0] = w0 * S[0] + w1 * S[1] + w2 * S[2];
-            N[i * 3 + 1] = w0 * S[1] + w1 * S[3] + w2 * S[4];
-            N[i * 3 + 2] = w0 * S[2] + w1 * S[4] + w2 * S[5];
-#pragma unroll
-            for (int j = 0; j < 3; ++j) lf += N[i * 3 + j] * Jc[i * 3 + j];
-        }
-        l_dlam = lnJ * tr;
-        l_dmu = lf * id * id - tr;
-        const double dc = det * ic, q0 = mu * id, q1 = (mu - lam * lnJ) * dc * ic, q2 = lam * tr * dc;
-#pragma unroll
-        for (int k = 0; k < 3; ++k)
-#pragma unroll
-            for (int i = 0; i < 3; ++i) {
-                const double cc = C[k * 3 + 0] * B[0 + i] + C[k * 3 + 1] * B[3 + i] + C[k * 3 + 2] * B[6 + i];
-                Q[k * 3 + i] = q0 * N[i * 3 + k] + q1 * cc + q2 * B[k * 3 + i];
-            }
-        return det;
-    }
-    double H[9], L[9], dP[9];
+    double H[9], L[9];  // L unscaled (W adj(J)) for the neo-Hookean term
 #pragma unroll
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
             H[i * 3 + j] = (G[i * 3 + 0] * A[0 * 3 + j] + G[i * 3 + 1] * A[1 * 3 + j] + G[i * 3 + 2] * A[2 * 3 + j]) * id;
-            L[i * 3 + j] = (W[i * 3 + 0] * A[0 * 3 + j] + W[i * 3 + 1] * A[1 * 3 + j] + W[i * 3 + 2] * A[2 * 3 + j]) * id;
+            L[i * 3 + j] = W[i * 3 + 0] * A[0 * 3 + j] + W[i * 3 + 1] * A[1 * 3 + j] + W[i * 3 + 2] * A[2 * 3 + j];
         }
+    if (MAT == kNeoHookean) {
+        const double Jm1 = det_ap_im1(H), mi = mu * id;
+        const double lnJ = log1p_nh(Jm1);
+        double E[6];  // F F^T - I, upper triangle
+        int t = 0;
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = i; j < 3; ++j)
+                E[t++] = H[i * 3 + j] + H[j * 3 + i] + (H[i * 3] * H[j * 3] + H[i * 3 + 1] * H[j * 3 + 1] + H[i * 3 + 2] * H[j * 3 + 2]);
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int i = 0; i < 3; ++i)
+                Q[k * 3 + i] = mi * (A[k * 3 + 0] * L[i * 3 + 0] + A[k * 3 + 1] * L[i * 3 + 1] + A[k * 3 + 2] * L[i * 3 + 2]);
+        double Jc[9], B[9], Y[9];
+#pragma unroll
+        for (int k = 0; k < 9; ++k) Jc[k] = J[k] + G[k];
+        adj3(Jc, B);
+        const double ic = id / (1.0 + Jm1);
+#pragma unroll
+        for (int i = 0; i < 3; ++i)
+#pragma unroll
+            for (int j = 0; j < 3; ++j) Y[i * 3 + j] = W[i * 3 + 0] * B[0 + j] + W[i * 3 + 1] * B[3 + j] + W[i * 3 + 2] * B[6 + j];
+        const double tr = (Y[0] + Y[4] + Y[8]) * ic;
+        l_dlam = lnJ * tr;
+        l_dmu = (E[0] * Y[0] + E[3] * Y[4] + E[5] * Y[8] + E[1] * (Y[1] + Y[3]) + E[2] * (Y[2] + Y[6]) + E[4] * (Y[5] + Y[7])) * ic;
+        const double dc = det * ic, q1 = (mu - lam * lnJ) * dc * ic, q2 = lam * tr * dc;
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const double by = B[k * 3 + 0] * Y[0 + i] + B[k * 3 + 1] * Y[3 + i] + B[k * 3 + 2] * Y[6 + i];
+                Q[k * 3 + i] += q1 * by + q2 * B[k * 3 + i];
+            }
+        return det;
+    }
+#pragma unroll
+    for (int k = 0; k < 9; ++k) L[k] *= id;
+    double dP[9];
     stress_vjp(MAT, lam, mu, H, L, dP, &l_dlam, &l_dmu);
 #pragma unroll
     for (int k = 0; k < 3; ++k)
@@ -2576,9 +2572,11 @@ __device__ __forceinline__ double hex_gauss_vjp(const double* J, const double* G
 
 // Hex8 VJP, four lanes per element as in k_hex8_force (its stages, groups and rounds); the
 // quad's lanes add their Gauss points' modulus sensitivities. On 64^3 neo-Hookean elements
-// with fields (B200): one thread per element (254 registers, spills) 117 us, quads 111 us
-// at three blocks per SM (168 registers; at four, 128 and more spills, the same; at two 128
-// us). Gather latency binds (FP64 pipe 44%).
+// with fields (B200): one thread per element (254 registers, spills) 117 us a launch under
+// ncu, quads 111 us at three blocks per SM (168 registers; at four, 128 and more spills, the
+// same; at two 128 us). In an adjoint run, by events, 107 us; 101 us with the shear-modulus
+// sensitivity from (W J^-1 J^-T) : Jc - tr, which loses its digits on thin elements (see
+// hex_gauss_vjp).
 constexpr int kHexVjpBlocks = 3;
 template <int MAT>
 __global__ void __launch_bounds__(kHexBlock, kHexVjpBlocks) k_hex8_vjp(GaussBlockDev b, const double4* __restrict__ X4,

@@ -1084,7 +1084,10 @@ constexpr int kHexBlocks = 4;  // sixteen warps per SM, 128 registers
 // most eight. From the second round on a warp has its connectivity at hand. Measured on
 // B200 at 128^3, neo-Hookean with fields (us per launch, 1 / 2 / 4 / 8 rounds): 497 / 480 /
 // 476 / 459. Fewer waves leave SMs empty: 20^3 linear elastic FP64 took
-// 7.7 us a step with one round, 8.1 with two and 11.7 with four.
+// 7.7 us a step with one round, 8.1 with two and 11.7 with four. The VJP kernel runs twelve
+// warps per SM and takes the same rounds; measured (us per launch, 1 / 2 / 4 / 6 / 8 rounds):
+// 20^3 10.7 / 12.1 / 17.9 / 23 / 29, 40^3 30.7 / 31.0 / 36.6 / 36.7 / 37.1, 64^3 109.6 / 106.9 /
+// 107.5 / 115 / 114.5, 100^3 397 / 383 / 379 / 375 / 374. The rule takes 1, 1, 4 and 8 there.
 inline int32_t hex_rounds(int64_t groups) { return static_cast<int32_t>(std::clamp<int64_t>(groups / (3 * 148 * 16), 1, 8)); }
 
 template <int MAT>

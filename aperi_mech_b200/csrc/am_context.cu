@@ -1357,8 +1357,9 @@ struct am_ctx {
         ck(cudaMemcpyAsync(xc, X4, N * sizeof(double4), cudaMemcpyDeviceToDevice, stream), "copy");
         ck(cudaMemsetAsync(lagr_inc, 0, N * sizeof(double4), stream), "memset");
         for (auto& b : blocks) {
-            ck(cudaMemsetAsync(b.hstate, 0, static_cast<size_t>(b.num_elems) * 9 * sizeof(double), stream), "memset");
-            if (b.href) ck(cudaMemsetAsync(b.href, 0, static_cast<size_t>(b.num_elems) * 9 * sizeof(double), stream), "memset");
+            const size_t bytes = static_cast<size_t>(am::lagr_stride(b.num_elems)) * 9 * sizeof(double);
+            ck(cudaMemsetAsync(b.hstate, 0, bytes, stream), "memset");
+            if (b.href) ck(cudaMemsetAsync(b.href, 0, bytes, stream), "memset");
         }
         lagr_steps = 0;
         lagr_rebased = false;
@@ -2045,7 +2046,7 @@ int am_finalize(am_ctx* ctx) {
             ctx->xc = dalloc<double4>(N, "current coordinates");
             ctx->lagr_inc = dalloc<double4>(N, "displacement increment");
             for (auto& b : ctx->blocks) {
-                const size_t n9 = static_cast<size_t>(std::max<int64_t>(b.num_elems, 1)) * 9;
+                const size_t n9 = static_cast<size_t>(am::lagr_stride(std::max<int64_t>(b.num_elems, 1))) * 9;
                 b.hstate = dalloc<double>(n9, "element H");
                 if (ctx->lagr == 2) b.href = dalloc<double>(n9, "reference H");
             }

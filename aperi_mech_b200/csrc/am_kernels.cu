@@ -1278,22 +1278,23 @@ __global__ void __launch_bounds__(128, 4) k_hex8_force_mixed(GaussBlockDev b, co
 // F_ref = I + Href: B F_ref and w / det F_ref. The element keeps one H (for Hex8 the last
 // Gauss point's, as the reference's element field), which is also every Gauss point's Href.
 // ---------------------------------------------------------------------------
-// The element H arrays are component-major (component k of element e at k E + e), so that a
-// warp's nine loads and stores are coalesced. They are written by the element kernel of the
-// previous step: read after the wait for the predecessor, with coherent loads.
-__device__ __forceinline__ void lagr_href(const GaussBlockDev& b, int64_t e, int32_t lagr, int rebase, bool own, double* hr) {
-    const int64_t E = b.num_elems;
+// The element H arrays are component-major (component k of element e at k lagr_stride + e), so
+// that a warp's nine loads and stores are coalesced. They are written by the element kernel of
+// the previous step: read after the wait for the predecessor, with coherent loads.
+__device__ __forceinline__ void lagr_href(const GaussBlockDev& b, int64_t e, int32_t lagr, int rebase, double* hr) {
+    const int64_t S = lagr_stride(b.num_elems);
     const double* src = (lagr == 1 || rebase) ? b.hstate : b.href;
 #pragma unroll
-    for (int k = 0; k < 9; ++k) hr[k] = __ldcg(src + k * E + e);
-    if (lagr == 2 && rebase && own) {
+    for (int k = 0; k < 9; ++k) hr[k] = __ldcg(src + k * S + e);
+    if (lagr == 2 && rebase) {
 #pragma unroll
-        for (int k = 0; k < 9; ++k) b.href[k * E + e] = hr[k];
+        for (int k = 0; k < 9; ++k) b.href[k * S + e] = hr[k];
     }
 }
 __device__ __forceinline__ void lagr_store_h(const GaussBlockDev& b, int64_t e, const double* H) {
+    const int64_t S = lagr_stride(b.num_elems);
 #pragma unroll
-    for (int k = 0; k < 9; ++k) b.hstate[k * b.num_elems + e] = H[k];
+    for (int k = 0; k < 9; ++k) b.hstate[k * S + e] = H[k];
 }
 
 // H = dH + Href + dH Href
@@ -1335,8 +1336,8 @@ __global__ void __launch_bounds__(128, 5) k_tet4_force_lagr(GaussBlockDev b, int
     pdl_trigger();
     const int64_t E = b.num_elems;
     const int64_t et = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    // chunked: lanes past the last tet run a copy of it (never summed, nothing kept) to
-    // reach the warp sum
+    // chunked: the block's lanes past the last tet run a copy of it (never summed) to reach the
+    // warp sum, each with an H of its own in the arrays' padding
     if (!CHUNKS && et >= E) return;
     const bool own = et < E;
     const int64_t e = own ? et : E - 1;
@@ -1352,7 +1353,7 @@ __global__ void __launch_bounds__(128, 5) k_tet4_force_lagr(GaussBlockDev b, int
     }
     pdl_wait();
     double dH[9], hr[9], H[9];
-    lagr_href(b, e, lagr, rebase, own, hr);
+    lagr_href(b, et, lagr, rebase, hr);
     const double4 x0 = ld_dep(XC + c.x), x1 = ld_dep(XC + c.y), x2 = ld_dep(XC + c.z), x3 = ld_dep(XC + c.w);
     const double4 u0 = ld_dep(INC + c.x), u1 = ld_dep(INC + c.y), u2 = ld_dep(INC + c.z), u3 = ld_dep(INC + c.w);
     const double J[9] = {x1.x - x0.x, x2.x - x0.x, x3.x - x0.x, x1.y - x0.y, x2.y - x0.y,
@@ -1369,7 +1370,7 @@ __global__ void __launch_bounds__(128, 5) k_tet4_force_lagr(GaussBlockDev b, int
 #pragma unroll
         for (int j = 0; j < 3; ++j) dH[i * 3 + j] = D[i * 3 + 0] * Ji[0 * 3 + j] + D[i * 3 + 1] * Ji[1 * 3 + j] + D[i * 3 + 2] * Ji[2 * 3 + j];
     lagr_compose(dH, hr, H);
-    if (keep && own) lagr_store_h(b, e, H);
+    if (keep) lagr_store_h(b, et, H);
     double lam, mu;
     element_lame(b, e, lam, mu);
     double P[9], Pm[9];
@@ -1434,7 +1435,7 @@ __global__ void __launch_bounds__(64) k_hex8_force_lagr(GaussBlockDev b, int32_t
     double lam, mu;
     element_lame(b, e, lam, mu);
     double hr[9];
-    lagr_href(b, e, lagr, rebase, true, hr);
+    lagr_href(b, e, lagr, rebase, hr);
     double R[3][8];
 #pragma unroll
     for (int i = 0; i < 3; ++i)

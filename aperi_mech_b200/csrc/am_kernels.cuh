@@ -27,6 +27,10 @@ enum StatusSlot { kStatusCode = 0, kStatusIndex = 1 };
 // logical slot order (block, then element / patch / entry). Writers map a logical
 // slot s of a block to its position with slot_pos[s] (block-local pointer).
 
+// Elements between two components of the updated / semi element H arrays: the element count
+// padded to whole 128-thread blocks, so that every lane of such a block has an entry.
+__host__ __device__ constexpr int64_t lagr_stride(int64_t num_elems) { return (num_elems + 127) / 128 * 128; }
+
 // Gauss-element block on the device.
 struct GaussBlockDev {
     int32_t kind;      // AM_TET4_GAUSS / AM_HEX8_GAUSS

@@ -332,26 +332,18 @@ struct Block {
     }
     // A chunked block's per-corner view for the kernels that write one value per element (or
     // patch) node: positions into the scratch array (allocated on first use) at 4 u + a, unit
-    // u and corner a. Per tet the identity; a split-hex patch p's node k (tets or cells) is
-    // corner a of half patch 2p + r (thread r writes nodes 1, 2, 4, 0 or 5, 6, 7, 3).
-    void ensure_corners() {
+    // u and corner a.
+    void ensure_corners(cudaStream_t stream) {
         const size_t n = static_cast<size_t>(4 * std::max<int64_t>(chunk_units, 1));
         if (!chunk_ident) {
-            std::vector<int32_t> id(n);
-            if (patched == 2) {
-                constexpr int kR[8] = {0, 0, 0, 1, 0, 1, 1, 1}, kA[8] = {3, 0, 1, 3, 2, 0, 1, 2};
-                for (int64_t p = 0; p < num_patches; ++p)
-                    for (int k = 0; k < 8; ++k) id[8 * p + k] = static_cast<int32_t>(4 * (2 * p + kR[k]) + kA[k]);
-            } else {
-                for (size_t k = 0; k < n; ++k) id[k] = static_cast<int32_t>(k);
-            }
             chunk_ident = dalloc<int32_t>(n, "chunk corner positions");
-            ck(cudaMemcpy(chunk_ident, id.data(), n * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
+            am::launch_chunk_corners(patched == 2 ? 1 : 0, 4 * chunk_units, chunk_ident, stream);
+            ck(cudaGetLastError(), "chunk corner positions");
         }
         if (!chunk_scratch) chunk_scratch = dalloc<double4>(n, "chunk corner values");
     }
-    am::GaussBlockDev gauss_corners() {
-        ensure_corners();
+    am::GaussBlockDev gauss_corners(cudaStream_t stream) {
+        ensure_corners(stream);
         am::GaussBlockDev g = gauss();
         g.slot_pos = chunk_ident;
         return g;
@@ -1107,7 +1099,7 @@ struct am_ctx {
     // most 32 subcells), which keeps L_s per subcell beside H_s.
     void prepare_vjp(const char* what) {
         for (auto& b : blocks) {
-            if (b.chunk_ptr) b.ensure_corners();
+            if (b.chunk_ptr) b.ensure_corners(stream);
             if (!b.group_ptr) continue;
             if (!b.gather) fail(AM_ESTATE, std::string(what) + " on F-bar cells needs the cell-stress form (cells of at most 32 subcells)");
             if (!b.vjp_lmat) b.vjp_lmat = dalloc<double>(std::max<int64_t>(9 * b.num_elems, 1), "F-bar VJP scratch");
@@ -2015,7 +2007,7 @@ int am_finalize(am_ctx* ctx) {
             for (auto& b : ctx->blocks) {
                 if (b.chunk_ptr) {
                     // allocates the scratch first: it is an argument of the launch below
-                    const am::GaussBlockDev corners = b.gauss_corners();
+                    const am::GaussBlockDev corners = b.gauss_corners(ctx->stream);
                     am::launch_gauss_volume_slots(corners, b.density, ctx->X4, b.chunk_scratch, ctx->stream);
                     am::launch_chunk_sum(b.gauss(), b.chunk_scratch, ctx->slots64, ctx->stream);
                     ctx->launches += 2;

@@ -353,6 +353,17 @@ __global__ void __launch_bounds__(256) k_chunk_positions(B b, int32_t* __restric
     }
 }
 
+// A chunked block's corner positions: per tet the identity; a split-hex patch p's node k (tets
+// or cells) is corner a of half patch 2p + r (thread r writes nodes 1, 2, 4, 0 or 5, 6, 7, 3).
+__global__ void __launch_bounds__(256) k_chunk_corners(int patches, int64_t n, int32_t* __restrict__ id) {
+    const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
+    if (t >= n) return;
+    const int k = static_cast<int>(t & 7);
+    const int corner = (0x30132012 >> (4 * (7 - k))) & 3;  // of nodes 0 .. 7: 3 0 1 3 2 0 1 2
+    const int half = (0xE8 >> k) & 1;                      // nodes 3, 5, 6, 7 are the second's
+    id[t] = static_cast<int32_t>(patches ? (t & ~int64_t{7}) + 4 * half + corner : t);
+}
+
 // Sums the chunk's entries per node and writes each node's slot once: a lane sums the runs
 // of its K sorted entries, a segmented inclusive scan over the lanes (fixed shuffle tree)
 // carries a run across lane boundaries, and the lane holding a node's last entry writes it.
@@ -4089,6 +4100,9 @@ void launch_hex6_patch_dx(const int32_t* patch_nodes, int64_t num_patches, const
     k_hex6_patch_dx<<<grid_for(num_patches, 256), 256, 0, stream>>>(patch_nodes, num_patches, X4, dx32, dx64);
 }
 
+void launch_chunk_corners(int patches, int64_t n, int32_t* id, cudaStream_t s) {
+    if (n > 0) k_chunk_corners<<<grid_for(n, 256), 256, 0, s>>>(patches, n, id);
+}
 void launch_chunk_positions(const GaussBlockDev& b, int32_t* out, cudaStream_t s) {
     if (b.chunk_units == 0) return;
     k_chunk_positions<4, GaussBlockDev><<<grid_for(b.chunk_units, 256), 256, 0, s>>>(b, out);

@@ -212,6 +212,8 @@ void launch_gauss_volume_slots(const GaussBlockDev& b, double density, const dou
 // Chunked blocks: per-corner values (scratch[nn e + a]) summed into the block's slots.
 void launch_chunk_sum(const GaussBlockDev& b, const double4* scratch, double4* slots, cudaStream_t s);
 void launch_chunk_sum(const CellBlockDev& b, const double4* scratch, double4* slots, cudaStream_t s);
+// Corner positions of a chunked block's n = 4 x units corners (patches: split-hex patch nodes).
+void launch_chunk_corners(int patches, int64_t n, int32_t* id, cudaStream_t s);
 // Chunked blocks: the run-end slot positions of every lane (at am_finalize, after the layout).
 void launch_chunk_positions(const GaussBlockDev& b, int32_t* out, cudaStream_t s);
 void launch_chunk_positions(const CellBlockDev& b, int32_t* out, cudaStream_t s);

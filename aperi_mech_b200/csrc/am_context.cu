@@ -223,8 +223,9 @@ struct Block {
     int32_t* cell_ptr = nullptr;
     int32_t* cell_nodes = nullptr;
     double* grads64 = nullptr;
-    float* grads32 = nullptr;   // not kept where unit32 is
-    float* unit32 = nullptr;    // half-patch tables of grouped four-entry cells (see CellBlockDev)
+    float* grads32 = nullptr;
+    // Half-patch tables of grouped four-entry cells (see CellBlockDev), in place of the arrays above
+    float* unit32 = nullptr;
     double* unit64 = nullptr;
     double* volumes = nullptr;
     int32_t max_entries = 0;
@@ -368,7 +369,6 @@ struct Block {
         c.max_entries = max_entries;
         c.patched = patched;
         c.num_patches = num_patches;
-        c.patch_first = patch_first;
         c.patch_nodes = patch_nodes;
         c.num_groups = num_groups;
         c.group_ptr = group_ptr;
@@ -834,6 +834,25 @@ struct am_ctx {
     // coupling (ExplicitSolver::ComputeForce, src/Solvers/Explicit.cpp:146-186) the blocks
     // see the physical displacement Psi U, their forces are gathered per node and scattered
     // to the generalized force Psi^T f, which the node kernels then read (f_given).
+    // The half-patch tables of a block of grouped element cells from the caller's CSR arrays,
+    // through a staging buffer of kUnitPatches patches. Such a block keeps the tables (160 bytes
+    // a cell, both precisions) and no CSR array (172 bytes).
+    static constexpr int64_t kUnitPatches = 1 << 16;
+    void upload_cell_units(Block& b, const double* grads, const double* volumes) {
+        const int64_t P = b.num_patches, S = std::min(P, kUnitPatches);
+        b.unit32 = dalloc<float>(80 * P, "half-patch gradients (FP32)");
+        b.unit64 = dalloc<double>(80 * P, "half-patch gradients");
+        std::unique_ptr<double, void (*)(double*)> stage(dalloc<double>(78 * S, "cell staging"), [](double* p) { cudaFree(p); });
+        for (int64_t q = 0; q < P; q += S) {
+            const int64_t n = std::min(S, P - q);
+            ck(cudaMemcpyAsync(stage.get(), grads + 72 * q, 72 * n * sizeof(double), cudaMemcpyHostToDevice, stream), "upload");
+            ck(cudaMemcpyAsync(stage.get() + 72 * S, volumes + 6 * q, 6 * n * sizeof(double), cudaMemcpyHostToDevice, stream), "upload");
+            am::launch_cell_units(stage.get(), stage.get() + 72 * S, q, n, P, b.unit32, b.unit64, stream);
+            ck(cudaGetLastError(), "half-patch gradients");
+        }
+        ck(cudaStreamSynchronize(stream), "synchronize");
+    }
+
     // The two-pass functions: Psi in (nodes) -> out (points); Psi^T in (points) -> out (nodes, N x 3).
     void rk_rows(const double4* in, double4* out) {
         if (rko_w)
@@ -1651,29 +1670,12 @@ int am_add_block(am_ctx* ctx, const am_block_desc* d, int32_t* block_id) {
                 }
                 for (int64_t s = 0; s < K; ++s)
                     if (d->cell_nodes[s] < 0 || d->cell_nodes[s] >= ctx->points()) fail(AM_EINVAL, "cell node index out of range");
-                std::vector<float> g32(K * 3);
-                for (int64_t s = 0; s < K * 3; ++s) {
+                for (int64_t s = 0; s < K * 3; ++s)
                     if (!std::isfinite(d->cell_grads[s])) fail(AM_EINVAL, "non-finite cell gradient");
-                    g32[s] = static_cast<float>(d->cell_grads[s]);
-                }
                 for (int64_t c = 0; c < E; ++c)
                     if (!(d->cell_volumes[c] > 0.0)) fail(AM_EINVAL, "cell volumes must be positive");
                 b.num_entries = K;
                 b.max_entries = maxlen;
-                b.cell_ptr = dalloc<int32_t>(E + 1, "cell ptr");
-                ck(cudaMemcpy(b.cell_ptr, ptr.data(), (E + 1) * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
-                if (K > 0) {
-                    b.cell_nodes = dalloc<int32_t>(K, "cell nodes");
-                    b.grads64 = dalloc<double>(K * 3, "cell grads");
-                    b.grads32 = dalloc<float>(K * 3, "cell grads fp32");
-                    ck(cudaMemcpy(b.cell_nodes, d->cell_nodes, K * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
-                    ck(cudaMemcpy(b.grads64, d->cell_grads, K * 3 * sizeof(double), cudaMemcpyHostToDevice), "upload");
-                    ck(cudaMemcpy(b.grads32, g32.data(), K * 3 * sizeof(float), cudaMemcpyHostToDevice), "upload");
-                }
-                if (E > 0) {
-                    b.volumes = dalloc<double>(E, "cell volumes");
-                    ck(cudaMemcpy(b.volumes, d->cell_volumes, E * sizeof(double), cudaMemcpyHostToDevice), "upload");
-                }
                 b.host_nodes.assign(d->cell_nodes, d->cell_nodes + K);
                 if (maxlen > 8 && ctx->cell_gather) {
                     b.host_cell_ptr = ptr;
@@ -1690,16 +1692,10 @@ int am_add_block(am_ctx* ctx, const am_block_desc* d, int32_t* block_id) {
                         b.patched = 2;
                         b.num_patches = P;
                         b.slot_count = 8 * P;
-                        b.patch_first = dalloc<int32_t>(P + 1, "patch offsets");
                         b.patch_nodes = dalloc<int32_t>(8 * P, "patch nodes");
-                        ck(cudaMemcpy(b.patch_first, tp.first.data(), (P + 1) * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
                         ck(cudaMemcpy(b.patch_nodes, tp.nodes.data(), 8 * P * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
                         b.host_nodes.assign(tp.nodes.begin(), tp.nodes.begin() + 8 * P);
-                        dfree(b.grads32);
-                        b.unit32 = dalloc<float>(80 * P, "half-patch gradients (FP32)");
-                        b.unit64 = dalloc<double>(80 * P, "half-patch gradients");
-                        am::launch_cell_units(b.grads64, b.volumes, P, b.unit32, b.unit64, ctx->stream);
-                        ck(cudaGetLastError(), "half-patch gradients");
+                        ctx->upload_cell_units(b, d->cell_grads, d->cell_volumes);
                         if (ctx->warp_chunks && ctx->lagr == 0) {
                             // warp chunks over the half patches, as for the split-hex tets
                             constexpr int kNode[2][4] = {{1, 2, 4, 0}, {5, 6, 7, 3}};
@@ -1710,6 +1706,24 @@ int am_add_block(am_ctx* ctx, const am_block_desc* d, int32_t* block_id) {
                             WarpChunks wc;
                             if (build_warp_chunks(half.data(), 2 * P, 4, wc)) upload_warp_chunks(b, wc, 2 * P);
                         }
+                    }
+                }
+                if (b.patched == 0) {
+                    b.cell_ptr = dalloc<int32_t>(E + 1, "cell ptr");
+                    ck(cudaMemcpy(b.cell_ptr, ptr.data(), (E + 1) * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
+                    if (K > 0) {
+                        std::vector<float> g32(K * 3);
+                        for (int64_t s = 0; s < K * 3; ++s) g32[s] = static_cast<float>(d->cell_grads[s]);
+                        b.cell_nodes = dalloc<int32_t>(K, "cell nodes");
+                        b.grads64 = dalloc<double>(K * 3, "cell grads");
+                        b.grads32 = dalloc<float>(K * 3, "cell grads fp32");
+                        ck(cudaMemcpy(b.cell_nodes, d->cell_nodes, K * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
+                        ck(cudaMemcpy(b.grads64, d->cell_grads, K * 3 * sizeof(double), cudaMemcpyHostToDevice), "upload");
+                        ck(cudaMemcpy(b.grads32, g32.data(), K * 3 * sizeof(float), cudaMemcpyHostToDevice), "upload");
+                    }
+                    if (E > 0) {
+                        b.volumes = dalloc<double>(E, "cell volumes");
+                        ck(cudaMemcpy(b.volumes, d->cell_volumes, E * sizeof(double), cudaMemcpyHostToDevice), "upload");
                     }
                 }
             } else {

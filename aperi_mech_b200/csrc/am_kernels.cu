@@ -1937,16 +1937,18 @@ __device__ __forceinline__ const float4* cell_units<float>(const CellBlockDev& b
 template <>
 __device__ __forceinline__ const double4* cell_units<double>(const CellBlockDev& b) { return reinterpret_cast<const double4*>(b.unit64); }
 
-// Set-up: the half-patch tables from the cells' CSR (CellBlockDev::unit32, unit64).
+// Set-up: units [first, first + count) of the half-patch tables (CellBlockDev::unit32, unit64)
+// from those units' cells' gradients and volumes in their own order.
 __global__ void __launch_bounds__(256) k_cell_units(const double* __restrict__ grads, const double* __restrict__ volumes,
-                                                    int64_t units, float4* __restrict__ u32, double4* __restrict__ u64) {
+                                                    int64_t first, int64_t count, int64_t units, float4* __restrict__ u32,
+                                                    double4* __restrict__ u64) {
     const int64_t t = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    const int64_t m = t / units, u = t % units;
+    const int64_t m = t / count, u = t % count;
     if (m >= 10) return;
     const double* g = m < 9 ? grads + 36 * u + 4 * m : volumes + 3 * u;
     const double4 v = make_double4(g[0], g[1], g[2], m < 9 ? g[3] : 0.0);
-    u64[m * units + u] = v;
-    u32[m * units + u] = make_float4(static_cast<float>(v.x), static_cast<float>(v.y), static_cast<float>(v.z), static_cast<float>(v.w));
+    u64[m * units + first + u] = v;
+    u32[m * units + first + u] = make_float4(static_cast<float>(v.x), static_cast<float>(v.y), static_cast<float>(v.z), static_cast<float>(v.w));
 }
 
 // Gradients and volumes come from the half-patch tables, whose vec4 loads are contiguous over
@@ -2838,16 +2840,6 @@ __global__ void __launch_bounds__(256) k_fbar_cell_vjp(CellBlockDev b, double* _
     store_theta(gmu, gk, s, -V * (ldm - 2.0 / 3.0 * ldl), -V * ldl, accumulate);
 }
 
-__device__ __forceinline__ void load_cell12(const double* p, double* g) {
-    const double2* q = reinterpret_cast<const double2*>(p);
-#pragma unroll
-    for (int k = 0; k < 6; ++k) {
-        const double2 v = __ldg(q + k);
-        g[2 * k] = v.x;
-        g[2 * k + 1] = v.y;
-    }
-}
-
 // VJP of the split-hex-grouped cells (FP64, one thread per patch): the cell VJP above
 // for the patch's six cells, summed per patch node.
 template <int MAT>
@@ -2860,13 +2852,15 @@ __global__ void __launch_bounds__(64) k_cell_hex6_vjp(CellBlockDev b, const doub
     double acc[8][3];
 #pragma unroll
     for (int a = 0; a < 8; ++a) acc[a][0] = acc[a][1] = acc[a][2] = 0.0;
-    const int64_t c0 = b.patch_first[p];
+    const int64_t units = 2 * b.num_patches;
 #pragma unroll 1
     for (int t = 0; t < 6; ++t) {
-        const int64_t c = c0 + t;
+        const int64_t c = 6 * p + t;
         const int ln[4] = {0, kRing[t], kRing[t + 1], 3};
-        double g[12];
-        load_cell12(b.grads64 + 12 * c, g);
+        const int r = t / 3, k3 = t % 3;
+        const double4* ut = cell_units<double>(b) + 2 * p + r;
+        const double4 ga = ld_once(ut + 3 * k3 * units), gb = ld_once(ut + (3 * k3 + 1) * units), gc = ld_once(ut + (3 * k3 + 2) * units);
+        const double g[12] = {ga.x, ga.y, ga.z, ga.w, gb.x, gb.y, gb.z, gb.w, gc.x, gc.y, gc.z, gc.w};
         double H[9], L[9];
 #pragma unroll
         for (int k = 0; k < 9; ++k) H[k] = L[k] = 0.0;
@@ -2887,7 +2881,7 @@ __global__ void __launch_bounds__(64) k_cell_hex6_vjp(CellBlockDev b, const doub
         element_lame(b, c, lam, mu);
         double dP[9], ldl, ldm;
         stress_vjp(MAT, lam, mu, H, L, dP, &ldl, &ldm);
-        const double V = b.volumes[c];
+        const double V = ld_once(reinterpret_cast<const double*>(ut + 9 * units) + k3);
 #pragma unroll
         for (int e = 0; e < 4; ++e)
 #pragma unroll
@@ -4087,12 +4081,12 @@ void launch_tet4_geometry(const int32_t* conn, int64_t num_elems, const double4*
     k_tet4_geometry<<<grid_for(num_elems, 256), 256, 0, s>>>(conn, num_elems, X4, geo32, geo64);
 }
 
-void launch_cell_units(const double* grads, const double* volumes, int64_t num_patches, float* unit32, double* unit64,
-                       cudaStream_t stream) {
-    if (num_patches <= 0) return;
-    k_cell_units<<<grid_for(20 * num_patches, 256), 256, 0, stream>>>(grads, volumes, 2 * num_patches,
-                                                                      reinterpret_cast<float4*>(unit32),
-                                                                      reinterpret_cast<double4*>(unit64));
+void launch_cell_units(const double* grads, const double* volumes, int64_t first_patch, int64_t count, int64_t num_patches,
+                       float* unit32, double* unit64, cudaStream_t stream) {
+    if (count <= 0) return;
+    k_cell_units<<<grid_for(20 * count, 256), 256, 0, stream>>>(grads, volumes, 2 * first_patch, 2 * count, 2 * num_patches,
+                                                                reinterpret_cast<float4*>(unit32),
+                                                                reinterpret_cast<double4*>(unit64));
 }
 void launch_hex6_patch_dx(const int32_t* patch_nodes, int64_t num_patches, const double4* X4, float* dx32,
                           double* dx64, cudaStream_t stream) {

@@ -110,10 +110,10 @@ struct CellBlockDev {
     int64_t num_entries;        // ptr[num_cells]
     int32_t max_entries;        // longest cell (selects thread- or group-per-cell)
     // Four-entry cells grouped as split hexes (patched == 2, see GaussBlockDev): cell
-    // patch_first[q] + t holds tet t of patch q; one slot per patch node.
+    // 6 q + t holds tet t of patch q; one slot per patch node; no ptr, nodes, gradients or
+    // volumes above.
     int32_t patched;
     int64_t num_patches;
-    const int32_t* patch_first;
     const int32_t* patch_nodes;
     // Such cells' gradients and volumes by half patch, as k_cell_hex6_force's threads read them:
     // unit 2q + r (cells 6q + 3r + k, k = 0, 1, 2) has vec4 number m at m * 2 num_patches + unit;
@@ -202,9 +202,10 @@ void launch_gauss_vjp(const GaussBlockDev& b, const double4* X4, const double4* 
 // Lm: scratch of 9 doubles per cell for F-bar blocks (null otherwise). Returns the launch count.
 int launch_cell_vjp(const CellBlockDev& b, const double4* U4, const double4* L4, double* Lm, double4* slots,
                     double* gmu, double* gkappa, int accumulate, cudaStream_t s);
-// The half-patch tables of four-entry cells grouped as split hexes (see CellBlockDev::unit32).
-void launch_cell_units(const double* grads, const double* volumes, int64_t num_patches, float* unit32, double* unit64,
-                       cudaStream_t stream);
+// Patches [first_patch, first_patch + count) of the half-patch tables of four-entry cells grouped
+// as split hexes (see CellBlockDev::unit32), from those patches' gradients and volumes.
+void launch_cell_units(const double* grads, const double* volumes, int64_t first_patch, int64_t count, int64_t num_patches,
+                       float* unit32, double* unit64, cudaStream_t stream);
 void launch_hex6_patch_dx(const int32_t* patch_nodes, int64_t num_patches, const double4* X4, float* dx32,
                           double* dx64, cudaStream_t stream);
 void launch_gauss_volume_slots(const GaussBlockDev& b, double density, const double4* X4, double4* slots,

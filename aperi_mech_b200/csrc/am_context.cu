@@ -2288,7 +2288,7 @@ int am_adjoint(am_ctx* ctx, int64_t nsteps, double dt, int32_t ckpt_every, int32
         const int64_t nseg = (nsteps + ckpt_every - 1) / ckpt_every;
         // Buffers (nodal double4 vectors) are cached on the context and reused while the
         // checkpoint layout and the sizes stay the same.
-        const int64_t n_vec = 3 * nseg + ckpt_every + 6;
+        const int64_t n_vec = 3 * nseg + ckpt_every + 5;
         const int64_t n_aux = 2 * ((E + 3) / 4) + (num_sensors + 7) / 8 + 2;
         if (ctx->adj_key[0] != n_vec || ctx->adj_key[1] != n_aux || ctx->adj_key[2] != ctx->N) {
             ck(cudaStreamSynchronize(ctx->stream), "synchronize");
@@ -2311,10 +2311,9 @@ int am_adjoint(am_ctx* ctx, int64_t nsteps, double dt, int32_t ckpt_every, int32
         for (int32_t k = 0; k < ckpt_every; ++k) seg[k] = B[3 * nseg + k];
         double4* UB = B[3 * nseg + ckpt_every + 0];
         double4* VB = B[3 * nseg + ckpt_every + 1];
-        double4* AB = B[3 * nseg + ckpt_every + 2];
-        double4* fin_u = B[3 * nseg + ckpt_every + 3];
-        double4* fin_v = B[3 * nseg + ckpt_every + 4];
-        double4* fin_a = B[3 * nseg + ckpt_every + 5];
+        double4* fin_u = B[3 * nseg + ckpt_every + 2];
+        double4* fin_v = B[3 * nseg + ckpt_every + 3];
+        double4* fin_a = B[3 * nseg + ckpt_every + 4];
         double* gm = reinterpret_cast<double*>(B[n_vec]);
         double* gk = gm + 4 * ((E + 3) / 4);
         int32_t* dsens = reinterpret_cast<int32_t*>(gk + 4 * ((E + 3) / 4));
@@ -2344,11 +2343,10 @@ int am_adjoint(am_ctx* ctx, int64_t nsteps, double dt, int32_t ckpt_every, int32
         // Cotangent of the loss.
         am::launch_zero4(UB, ctx->N, st);
         am::launch_zero4(VB, ctx->N, st);
-        am::launch_zero4(AB, ctx->N, st);
         am::launch_sensor_seed(ctx->U4, num_sensors, dsens, UB, dloss, st);
-        ctx->launches += 4;
+        ctx->launches += 3;
         const am::NodeDev nd = ctx->node_dev();
-        am::launch_adj_prep(nd, ctx->table, nsteps - 1, VB, AB, ctx->L4, st);
+        am::launch_adj_prep(nd, ctx->table, nsteps - 1, VB, ctx->L4, st);
         ++ctx->launches;
         // Reverse pass, one segment at a time: recompute the segment's displacements
         // from its checkpoint, then transpose its steps in reverse order.

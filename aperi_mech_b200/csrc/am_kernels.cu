@@ -937,45 +937,37 @@ constexpr double kHexR = 0.26794919243112270647;   // (1 - c) / (1 + c) = 2 - sq
 constexpr double kHexScale = 0.31100423396407310780;  // (1 + c)^2 / 8: derivative = kHexScale x raw
 constexpr int kHexBlock = 128;
 
-template <typename T>
 struct HexPair {
-    T a, b;  // at the xi = -1 and xi = +1 nodes (or Gauss points) of the lane
+    double a, b;  // at the xi = -1 and xi = +1 nodes (or Gauss points) of the lane
 };
-__device__ __forceinline__ HexPair<double> hp_fma(double k, const HexPair<double>& x, const HexPair<double>& y) {
+__device__ __forceinline__ HexPair hp_fma(double k, const HexPair& x, const HexPair& y) {
     return {fma(k, x.a, y.a), fma(k, x.b, y.b)};
 }
-template <typename T>
-__device__ __forceinline__ HexPair<T> hp_xor(const HexPair<T>& x, int mask) {
+__device__ __forceinline__ HexPair hp_xor(const HexPair& x, int mask) {
     return {__shfl_xor_sync(kFull, x.a, mask), __shfl_xor_sync(kFull, x.b, mask)};
 }
 // The xi interpolation (its own transpose).
-template <typename T>
-__device__ __forceinline__ HexPair<T> hp_interp(const HexPair<T>& x) {
-    const T r = T(kHexR);
-    return {fma(r, x.b, x.a), fma(r, x.a, x.b)};
+__device__ __forceinline__ HexPair hp_interp(const HexPair& x) {
+    return {fma(kHexR, x.b, x.a), fma(kHexR, x.a, x.b)};
 }
-__device__ __forceinline__ HexPair<double> hp_scale(double k, const HexPair<double>& x) { return {k * x.a, k * x.b}; }
+__device__ __forceinline__ HexPair hp_scale(double k, const HexPair& x) { return {k * x.a, k * x.b}; }
 
 // Raw derivatives of one component at the lane's two Gauss points: d0 (xi, the same at
 // both), d1 (eta), d2 (zeta).
-template <typename T>
-__device__ __forceinline__ void hex_derivatives(const HexPair<T>& v, T& d0, HexPair<T>& d1, HexPair<T>& d2) {
-    const T r = T(kHexR);
-    const HexPair<T> q = hp_xor(v, 1);
-    const HexPair<T> D = hp_fma(T(-1), q, v), I = hp_fma(r, q, v);
-    const HexPair<T> Dz = hp_xor(D, 2), Iz = hp_xor(I, 2);
-    d1 = hp_interp(hp_fma(r, Dz, D));
-    d2 = hp_interp(hp_fma(T(-1), Iz, I));
-    d0 = fma(r, Iz.b - Iz.a, I.b - I.a);
+__device__ __forceinline__ void hex_derivatives(const HexPair& v, double& d0, HexPair& d1, HexPair& d2) {
+    const HexPair q = hp_xor(v, 1);
+    const HexPair D = hp_fma(-1.0, q, v), I = hp_fma(kHexR, q, v);
+    const HexPair Dz = hp_xor(D, 2), Iz = hp_xor(I, 2);
+    d1 = hp_interp(hp_fma(kHexR, Dz, D));
+    d2 = hp_interp(hp_fma(-1.0, Iz, I));
+    d0 = fma(kHexR, Iz.b - Iz.a, I.b - I.a);
 }
 // The transpose: z the xi terms summed over the two points, y1 and y2 the eta and zeta terms.
-template <typename T>
-__device__ __forceinline__ HexPair<T> hex_transpose(T z, const HexPair<T>& q1, const HexPair<T>& q2) {
-    const T r = T(kHexR);
-    const HexPair<T> j0{-z, z}, y1 = hp_interp(q1), y2 = hp_interp(q2);
-    const HexPair<T> w = hp_fma(T(1), hp_xor(hp_fma(-r, j0, y2), 2), hp_fma(T(1), j0, y2));
-    const HexPair<T> v = hp_fma(-r, hp_xor(y1, 2), y1);
-    return hp_fma(T(1), hp_xor(hp_fma(-r, w, v), 1), hp_fma(T(1), w, v));
+__device__ __forceinline__ HexPair hex_transpose(double z, const HexPair& q1, const HexPair& q2) {
+    const HexPair j0{-z, z}, y1 = hp_interp(q1), y2 = hp_interp(q2);
+    const HexPair w = hp_fma(1.0, hp_xor(hp_fma(-kHexR, j0, y2), 2), hp_fma(1.0, j0, y2));
+    const HexPair v = hp_fma(-kHexR, hp_xor(y1, 2), y1);
+    return hp_fma(1.0, hp_xor(hp_fma(-kHexR, w, v), 1), hp_fma(1.0, w, v));
 }
 
 // Q = adj(J) P^T at a Gauss point from J and the displacement gradient G
@@ -985,7 +977,7 @@ template <int MAT>
 __device__ __forceinline__ bool hex_gauss_q(const double* J, const double* G, double lam, double mu, double sig, double* Q) {
     double A[9];
     adj3(J, A);
-    const double det = vfma(J[2], A[6], vfma(J[1], A[3], vmul(J[0], A[0])));
+    const double det = fma(J[2], A[6], fma(J[1], A[3], J[0] * A[0]));
     bool ok = sig * det > 0.0;
     const double id = 1.0 / det;
     double H[9];
@@ -993,23 +985,22 @@ __device__ __forceinline__ bool hex_gauss_q(const double* J, const double* G, do
     for (int i = 0; i < 3; ++i)
 #pragma unroll
         for (int j = 0; j < 3; ++j)
-            H[i * 3 + j] = vmul(vfma(G[i * 3 + 2], A[6 + j], vfma(G[i * 3 + 1], A[3 + j], vmul(G[i * 3 + 0], A[j]))), id);
-    const double m = mu;
+            H[i * 3 + j] = fma(G[i * 3 + 2], A[6 + j], fma(G[i * 3 + 1], A[3 + j], G[i * 3 + 0] * A[j])) * id;
     if (MAT == kNeoHookean) {
         // Q = adj(J) P^T with P = tau F^-T and F = (J + G) J^-1 is adj(J + G) tau / det F
         // (the scale of J and G cancels): no F^-1 and no P.
         double lln, iJ;
         ok = nh_scalars(H, lam, lln, iJ) && ok;
-        const double sm = vmul(m, iJ), sl = vmul(lln, iJ);
+        const double sm = mu * iJ, sl = lln * iJ;
         double ts[9];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int j = i; j < 3; ++j) {
-                double t = vadd(H[i * 3 + j], H[j * 3 + i]);
+                double t = H[i * 3 + j] + H[j * 3 + i];
 #pragma unroll
-                for (int k = 0; k < 3; ++k) t = vfma(H[i * 3 + k], H[j * 3 + k], t);
-                t = i == j ? vfma(sm, t, sl) : vmul(sm, t);
+                for (int k = 0; k < 3; ++k) t = fma(H[i * 3 + k], H[j * 3 + k], t);
+                t = i == j ? fma(sm, t, sl) : sm * t;
                 ts[i * 3 + j] = ts[j * 3 + i] = t;
             }
         double Jc[9], Ac[9];
@@ -1020,19 +1011,18 @@ __device__ __forceinline__ bool hex_gauss_q(const double* J, const double* G, do
         for (int k = 0; k < 3; ++k)
 #pragma unroll
             for (int i = 0; i < 3; ++i)
-                Q[k * 3 + i] = vfma(Ac[k * 3 + 2], ts[6 + i], vfma(Ac[k * 3 + 1], ts[3 + i], vmul(Ac[k * 3 + 0], ts[i])));
+                Q[k * 3 + i] = fma(Ac[k * 3 + 2], ts[6 + i], fma(Ac[k * 3 + 1], ts[3 + i], Ac[k * 3 + 0] * ts[i]));
         return ok;
     }
     double P[9];
-    const double l = lam;
     if (MAT == kLinearElastic) {
-        const double tr = vmul(l, vadd(vadd(H[0], H[4]), H[8]));
+        const double tr = lam * (H[0] + H[4] + H[8]);
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int j = i; j < 3; ++j) {
-                const double e = vadd(H[i * 3 + j], H[j * 3 + i]);
-                P[i * 3 + j] = P[j * 3 + i] = i == j ? vfma(m, e, tr) : vmul(m, e);
+                const double e = H[i * 3 + j] + H[j * 3 + i];
+                P[i * 3 + j] = P[j * 3 + i] = i == j ? fma(mu, e, tr) : mu * e;
             }
     } else {
         // 2E = H + H^T + H^T H, S = lambda/2 tr(2E) I + mu 2E, P = S + H S
@@ -1041,26 +1031,26 @@ __device__ __forceinline__ bool hex_gauss_q(const double* J, const double* G, do
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int j = i; j < 3; ++j) {
-                double e = vadd(H[i * 3 + j], H[j * 3 + i]);
+                double e = H[i * 3 + j] + H[j * 3 + i];
 #pragma unroll
-                for (int k = 0; k < 3; ++k) e = vfma(H[k * 3 + i], H[k * 3 + j], e);
+                for (int k = 0; k < 3; ++k) e = fma(H[k * 3 + i], H[k * 3 + j], e);
                 E[i * 3 + j] = E[j * 3 + i] = e;
             }
-        const double tr = vmul(0.5 * lam, vadd(vadd(E[0], E[4]), E[8]));
+        const double tr = 0.5 * lam * (E[0] + E[4] + E[8]);
         double S[9];
 #pragma unroll
-        for (int k = 0; k < 9; ++k) S[k] = k % 4 == 0 ? vfma(m, E[k], tr) : vmul(m, E[k]);
+        for (int k = 0; k < 9; ++k) S[k] = k % 4 == 0 ? fma(mu, E[k], tr) : mu * E[k];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
 #pragma unroll
             for (int j = 0; j < 3; ++j)
-                P[i * 3 + j] = vfma(H[i * 3 + 2], S[6 + j], vfma(H[i * 3 + 1], S[3 + j], vfma(H[i * 3 + 0], S[j], S[i * 3 + j])));
+                P[i * 3 + j] = fma(H[i * 3 + 2], S[6 + j], fma(H[i * 3 + 1], S[3 + j], fma(H[i * 3 + 0], S[j], S[i * 3 + j])));
     }
 #pragma unroll
     for (int k = 0; k < 3; ++k)
 #pragma unroll
         for (int i = 0; i < 3; ++i)
-            Q[k * 3 + i] = vfma(A[k * 3 + 2], P[i * 3 + 2], vfma(A[k * 3 + 1], P[i * 3 + 1], vmul(A[k * 3 + 0], P[i * 3 + 0])));
+            Q[k * 3 + i] = fma(A[k * 3 + 2], P[i * 3 + 2], fma(A[k * 3 + 1], P[i * 3 + 1], A[k * 3 + 0] * P[i * 3 + 0]));
     return ok;
 }
 
@@ -1072,7 +1062,7 @@ __device__ __forceinline__ int2 hex_edge_pair(const int32_t* per_node, int64_t e
 }
 
 // A lane's two nodes and the element's node 0 of a nodal field, as loaded, and the two values
-// relative to node 0 (FP64 differences, then T).
+// relative to node 0.
 struct HexRaw {
     double4 o, a, b;
     template <bool DEP>
@@ -1081,11 +1071,10 @@ struct HexRaw {
         a = DEP ? ld_dep(A + n.x) : ld_ro4(A + n.x);
         b = DEP ? ld_dep(A + n.y) : ld_ro4(A + n.y);
     }
-    template <typename T>
-    __device__ __forceinline__ void rel(HexPair<T>* v) const {
-        v[0] = {T(a.x - o.x), T(b.x - o.x)};
-        v[1] = {T(a.y - o.y), T(b.y - o.y)};
-        v[2] = {T(a.z - o.z), T(b.z - o.z)};
+    __device__ __forceinline__ void rel(HexPair* v) const {
+        v[0] = {a.x - o.x, b.x - o.x};
+        v[1] = {a.y - o.y, b.y - o.y};
+        v[2] = {a.z - o.z, b.z - o.z};
     }
 };
 
@@ -1130,17 +1119,17 @@ __global__ void __launch_bounds__(kHexBlock, kHexBlocks) k_hex8_force(GaussBlock
         U.load<true>(U4, n0, n);
         // the next group's connectivity travels while this one is computed
         if (g + W < last) n = hex_edge_pair(b.conn, elem(g + W), p);
-        HexPair<double> x[3], u[3];
-        X.rel<double>(x);
-        U.rel<double>(u);
+        HexPair x[3], u[3];
+        X.rel(x);
+        U.rel(u);
         double J0[3], G0[3];
-        HexPair<double> J1[3], J2[3], G1[3], G2[3];
+        HexPair J1[3], J2[3], G1[3], G2[3];
 #pragma unroll
         for (int i = 0; i < 3; ++i) hex_derivatives(x[i], J0[i], J1[i], J2[i]);
 #pragma unroll
         for (int i = 0; i < 3; ++i) hex_derivatives(u[i], G0[i], G1[i], G2[i]);
         double z[3];
-        HexPair<double> q1[3], q2[3];
+        HexPair q1[3], q2[3];
         bool ok = true;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
@@ -1170,7 +1159,7 @@ __global__ void __launch_bounds__(kHexBlock, kHexBlocks) k_hex8_force(GaussBlock
         }
         const bool valid = 8 * g + (lane >> 2) < E;
         if (!ok && valid) flag(status, AM_ENONPOS_J, e);
-        HexPair<double> f[3];
+        HexPair f[3];
 #pragma unroll
         for (int i = 0; i < 3; ++i)
             f[i] = hp_scale(-sig * kHexScale * kHexScale * kHexScale, hex_transpose(z[i], q1[i], q2[i]));
@@ -2624,18 +2613,18 @@ __global__ void __launch_bounds__(kHexBlock, kHexVjpBlocks) k_hex8_vjp(GaussBloc
         V.load<true>(L4, n0, n);
         if (g + NW < last) n = hex_edge_pair(b.conn, elem(g + NW), p);
         double J0[3], G0[3], W0[3];
-        HexPair<double> v[3], J1[3], J2[3], G1[3], G2[3], W1[3], W2[3];
-        X.rel<double>(v);
+        HexPair v[3], J1[3], J2[3], G1[3], G2[3], W1[3], W2[3];
+        X.rel(v);
 #pragma unroll
         for (int i = 0; i < 3; ++i) hex_derivatives(v[i], J0[i], J1[i], J2[i]);
-        U.rel<double>(v);
+        U.rel(v);
 #pragma unroll
         for (int i = 0; i < 3; ++i) hex_derivatives(v[i], G0[i], G1[i], G2[i]);
-        V.rel<double>(v);
+        V.rel(v);
 #pragma unroll
         for (int i = 0; i < 3; ++i) hex_derivatives(v[i], W0[i], W1[i], W2[i]);
         double z[3], tm = 0.0, tk = 0.0;
-        HexPair<double> q1[3], q2[3];
+        HexPair q1[3], q2[3];
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             double J[9], G[9], W[9], Q[9], ldl, ldm;
@@ -2668,7 +2657,7 @@ __global__ void __launch_bounds__(kHexBlock, kHexVjpBlocks) k_hex8_vjp(GaussBloc
             }
         }
         const bool valid = 8 * g + (lane >> 2) < E;
-        HexPair<double> f[3];
+        HexPair f[3];
 #pragma unroll
         for (int i = 0; i < 3; ++i) f[i] = hp_scale(-s3 * sig, hex_transpose(z[i], q1[i], q2[i]));
 #pragma unroll
@@ -3300,19 +3289,18 @@ __global__ void __launch_bounds__(kNodeBlock, sizeof(S) == 4 && BATCH == 8 ? 7 :
     node_update(nd, i, fx, fy, fz, m, w, vh, u0, sc, table, step, advance, U4, V4, A4, u_copy, status, rebase);
 }
 
-// Reverse of the acceleration step: lam = Ma (abar + h vbar) / m, the cotangent
-// of the internal force at step `step`.
+// Reverse of the last acceleration step: lam = Ma h vbar / m, the cotangent of the internal
+// force at step `step` (nothing reads the final acceleration, so abar = 0).
 __global__ void k_adj_prep(NodeDev nd, const StepParams* __restrict__ table, int64_t step,
-                           const double4* __restrict__ VB, const double4* __restrict__ AB, double4* __restrict__ L4) {
+                           const double4* __restrict__ VB, double4* __restrict__ L4) {
     const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (i >= nd.num_nodes) return;
     const StepParams& P = table[step];
     const double m = nd.mass[i];
     double mx, my, mz;
     free_mask(nd.bcword[i], P.aact, mx, my, mz);
-    const double4 vb = VB[i], ab = AB[i];
-    L4[i] = make_double4(mx * (ab.x + P.half * vb.x) / m, my * (ab.y + P.half * vb.y) / m,
-                         mz * (ab.z + P.half * vb.z) / m, 0.0);
+    const double4 vb = VB[i];
+    L4[i] = make_double4(mx * (P.half * vb.x) / m, my * (P.half * vb.y) / m, mz * (P.half * vb.z) / m, 0.0);
 }
 
 // Reverse of the rest of step `step` given g = (dF/du)^T lam in the slots; then
@@ -4156,26 +4144,25 @@ inline bool gather_batch8(const NodeDev& nd, int mixed) {
     return bytes <= (int64_t{64} << 20);
 }
 
+// A node kernel's instance for slots of type S by the lanes per node (lpn) and batch (b8).
+#define AM_NODE_LANES_PDL(KERNEL, S, ...)                                                             \
+    do {                                                                                              \
+        const vec4_t<S>* sl = static_cast<const vec4_t<S>*>(slots);                                   \
+        if (lpn == 8) launch_pdl(KERNEL<S, 4, 8>, grid, kNodeBlock, s, nd, sl, __VA_ARGS__);          \
+        else if (lpn == 4) launch_pdl(KERNEL<S, 2, 4>, grid, kNodeBlock, s, nd, sl, __VA_ARGS__);     \
+        else if (lpn == 2) launch_pdl(KERNEL<S, 4, 2>, grid, kNodeBlock, s, nd, sl, __VA_ARGS__);     \
+        else if (b8) launch_pdl(KERNEL<S, 8, 1>, grid, kNodeBlock, s, nd, sl, __VA_ARGS__);           \
+        else launch_pdl(KERNEL<S, 4, 1>, grid, kNodeBlock, s, nd, sl, __VA_ARGS__);                   \
+    } while (0)
 #define AM_NODE_DISPATCH_PDL(KERNEL, ...)                                                             \
     do {                                                                                              \
-        const int lpn = node_lanes(nd, mixed);                                                               \
+        const int lpn = node_lanes(nd, mixed);                                                        \
         const unsigned grid = grid_for((nd.subset_nodes ? nd.subset_count : nd.num_nodes) * lpn, kNodeBlock); \
         const bool b8 = gather_batch8(nd, mixed);                                                     \
-        if (mixed) {                                                                                  \
-            const float4* sl = static_cast<const float4*>(slots);                                     \
-            if (lpn == 8) launch_pdl(KERNEL<float, 4, 8>, grid, kNodeBlock, s, nd, sl, __VA_ARGS__);   \
-            else if (lpn == 4) launch_pdl(KERNEL<float, 2, 4>, grid, kNodeBlock, s, nd, sl, __VA_ARGS__); \
-            else if (lpn == 2) launch_pdl(KERNEL<float, 4, 2>, grid, kNodeBlock, s, nd, sl, __VA_ARGS__); \
-            else if (b8) launch_pdl(KERNEL<float, 8, 1>, grid, kNodeBlock, s, nd, sl, __VA_ARGS__);    \
-            else launch_pdl(KERNEL<float, 4, 1>, grid, kNodeBlock, s, nd, sl, __VA_ARGS__);            \
-        } else {                                                                                      \
-            const double4* sl = static_cast<const double4*>(slots);                                   \
-            if (lpn == 8) launch_pdl(KERNEL<double, 4, 8>, grid, kNodeBlock, s, nd, sl, __VA_ARGS__);  \
-            else if (lpn == 4) launch_pdl(KERNEL<double, 2, 4>, grid, kNodeBlock, s, nd, sl, __VA_ARGS__); \
-            else if (lpn == 2) launch_pdl(KERNEL<double, 4, 2>, grid, kNodeBlock, s, nd, sl, __VA_ARGS__); \
-            else if (b8) launch_pdl(KERNEL<double, 8, 1>, grid, kNodeBlock, s, nd, sl, __VA_ARGS__);   \
-            else launch_pdl(KERNEL<double, 4, 1>, grid, kNodeBlock, s, nd, sl, __VA_ARGS__);           \
-        }                                                                                             \
+        if (mixed)                                                                                    \
+            AM_NODE_LANES_PDL(KERNEL, float, __VA_ARGS__);                                            \
+        else                                                                                          \
+            AM_NODE_LANES_PDL(KERNEL, double, __VA_ARGS__);                                           \
     } while (0)
 
 #define AM_NODE_DISPATCH(KERNEL, ...)                                                                 \
@@ -4242,15 +4229,17 @@ void launch_node_step(const NodeDev& nd, int mixed, const void* slots, const Ste
     AM_NODE_DISPATCH_PDL(k_node_step, table, step, advance, U4, V4, A4, u_copy, status, rebase);
 }
 
-void launch_adj_prep(const NodeDev& nd, const StepParams* table, int64_t step, const double4* VB, const double4* AB,
-                     double4* L4, cudaStream_t s) {
-    k_adj_prep<<<grid_for(nd.num_nodes, 256), 256, 0, s>>>(nd, table, step, VB, AB, L4);
+void launch_adj_prep(const NodeDev& nd, const StepParams* table, int64_t step, const double4* VB, double4* L4,
+                     cudaStream_t s) {
+    k_adj_prep<<<grid_for(nd.num_nodes, 256), 256, 0, s>>>(nd, table, step, VB, L4);
 }
 
 void launch_adj_update(const NodeDev& nd, const void* slots, const StepParams* table, int64_t step, double4* UB,
                        double4* VB, double4* L4, cudaStream_t s) {
-    const int mixed = 0;
-    AM_NODE_DISPATCH_PDL(k_adj_update, table, step, UB, VB, L4);
+    const int lpn = node_lanes(nd, 0);
+    const unsigned grid = grid_for(nd.num_nodes * lpn, kNodeBlock);
+    const bool b8 = gather_batch8(nd, 0);
+    AM_NODE_LANES_PDL(k_adj_update, double, table, step, UB, VB, L4);
 }
 
 void launch_sensor_seed(const double4* U4, int32_t num_sensors, const int32_t* sensors, double4* UB, double* loss,

@@ -243,8 +243,8 @@ void launch_node_step(const NodeDev& nd, int mixed, const void* slots, const Ste
                       int advance, double4* U4, double4* V4, double4* A4, double4* u_copy, int* status,
                       cudaStream_t s, int rebase = 0);
 // Adjoint node kernels.
-void launch_adj_prep(const NodeDev& nd, const StepParams* table, int64_t step, const double4* VB, const double4* AB,
-                     double4* L4, cudaStream_t s);
+void launch_adj_prep(const NodeDev& nd, const StepParams* table, int64_t step, const double4* VB, double4* L4,
+                     cudaStream_t s);
 void launch_adj_update(const NodeDev& nd, const void* slots, const StepParams* table, int64_t step, double4* UB,
                        double4* VB, double4* L4, cudaStream_t s);
 // Power method for the stable time increment (PowerMethodProcessor.h:196-330):

@@ -157,12 +157,6 @@ __device__ __forceinline__ double stress(int32_t mat, T lambda, T mu, const T* H
     return 1.0;
 }
 
-// Fused operations written out (Hex8 quads), so that their order does not depend on the
-// compiler's contraction.
-__device__ __forceinline__ double vadd(double x, double y) { return x + y; }
-__device__ __forceinline__ double vmul(double x, double y) { return x * y; }
-__device__ __forceinline__ double vfma(double x, double y, double z) { return fma(x, y, z); }
-
 // Neo-Hookean log J and 1 / J (the two scalars its stress needs) as in nh_kirchhoff; returns
 // whether J is positive.
 __device__ __forceinline__ bool nh_scalars(const double* H, double lambda, double& lam_lnJ, double& iJ) {

@@ -10,6 +10,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <limits>
 #include <memory>
 #include <stdexcept>
 #include <type_traits>
@@ -2709,7 +2710,9 @@ int am_set_rk_functions(am_ctx* ctx, const int64_t* nbr_ptr, const int32_t* nbr,
                               int32_t*& idx, int64_t& n_oct) {
                 const OctetRows o = octet_rows(count, ptr, part, nullptr, nullptr, 8, true);
                 std::vector<double> h(o.src.size());
-                for (size_t q = 0; q < h.size(); ++q) h[q] = o.src[q] < 0 ? pad64() : w[o.src[q]];
+                // a NaN weight, whatever its bits, as the plain NaN: padding is a NaN of its own
+                const auto weight = [&](int32_t e) { return std::isnan(w[e]) ? std::numeric_limits<double>::quiet_NaN() : w[e]; };
+                for (size_t q = 0; q < h.size(); ++q) h[q] = o.src[q] < 0 ? pad64() : weight(o.src[q]);
                 up(iptr, o.index_ptr.data(), static_cast<int64_t>(o.index_ptr.size()), "function octet index offsets");
                 up(idx, o.index.data(), static_cast<int64_t>(o.index.size()), "function octet indices");
                 n_oct = static_cast<int64_t>(o.ptr.size()) - 1;

@@ -99,6 +99,14 @@ void nccl_check(ncclResult_t r, const char* what) {
     }
 }
 
+// Copies host data to the device and waits for its arrival. A copy from pageable memory may
+// return with its last part still on the way, ordered on the default stream only, and the
+// context's own stream does not wait for that one.
+void h2d(void* dst, const void* src, size_t bytes, const char* what) {
+    ck(cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice), what);
+    ck(cudaStreamSynchronize(cudaStreamLegacy), what);
+}
+
 // Octet rows of the cell-stress form: items 8o .. 8o + 7 (cells, or nodes), item j with
 // entries ptr[j] .. ptr[j+1] whose partners (node, or cell) ascend. Rows are aligned by
 // offset (partner minus item, or their anchors': on a locality-numbered mesh consecutive
@@ -527,8 +535,8 @@ struct Block {
             }
             r32 = dalloc<float4>(std::max<size_t>(R, 1), what);
             r64 = dalloc<double4>(std::max<size_t>(R, 1), what);
-            ck(cudaMemcpy(r32, h32.data(), R * sizeof(float4), cudaMemcpyHostToDevice), "upload");
-            ck(cudaMemcpy(r64, h64.data(), R * sizeof(double4), cudaMemcpyHostToDevice), "upload");
+            h2d(r32, h32.data(), R * sizeof(float4), "upload");
+            h2d(r64, h64.data(), R * sizeof(double4), "upload");
         };
         records(co, cperm, cpart, orec32, orec64, "cell octet records");
         records(no, tperm, tpart, nrec32, nrec64, "node octet records");
@@ -544,9 +552,9 @@ struct Block {
         c_ref = dalloc<int32_t>(std::max<int64_t>(E, 1), "cell reference nodes");
         cmat32 = dalloc<float>(std::max<int64_t>(9 * E, 1), "cell matrices (FP32)");
         cmat64 = dalloc<double>(std::max<int64_t>(9 * E, 1), "cell matrices");
-        ck(cudaMemcpy(o_ptr, co.ptr.data(), co.ptr.size() * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
-        ck(cudaMemcpy(n_ptr, no.ptr.data(), no.ptr.size() * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
-        ck(cudaMemcpy(c_ref, ref.data(), E * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
+        h2d(o_ptr, co.ptr.data(), co.ptr.size() * sizeof(int32_t), "upload");
+        h2d(n_ptr, no.ptr.data(), no.ptr.size() * sizeof(int32_t), "upload");
+        h2d(c_ref, ref.data(), E * sizeof(int32_t), "upload");
         t_count = T;
         host_nodes = std::move(nodes);
         gather = true;
@@ -563,9 +571,9 @@ void upload_warp_chunks(Block& b, WarpChunks& wc, int64_t units) {
     b.chunk_ptr = dalloc<int32_t>(C + 1, "chunk offsets");
     b.chunk_code = dalloc<uint32_t>(words, "chunk entry codes");
     b.chunk_rank = dalloc<uint32_t>(words, "chunk entry ranks");
-    ck(cudaMemcpy(b.chunk_ptr, wc.ptr.data(), (C + 1) * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
-    ck(cudaMemcpy(b.chunk_code, wc.code.data(), words * sizeof(uint32_t), cudaMemcpyHostToDevice), "upload");
-    ck(cudaMemcpy(b.chunk_rank, wc.rank.data(), words * sizeof(uint32_t), cudaMemcpyHostToDevice), "upload");
+    h2d(b.chunk_ptr, wc.ptr.data(), (C + 1) * sizeof(int32_t), "upload");
+    h2d(b.chunk_code, wc.code.data(), words * sizeof(uint32_t), "upload");
+    h2d(b.chunk_rank, wc.rank.data(), words * sizeof(uint32_t), "upload");
     b.slot_count = static_cast<int64_t>(wc.nodes.size());
     b.host_nodes = std::move(wc.nodes);
     b.chunk_units = units;
@@ -996,7 +1004,7 @@ struct am_ctx {
                 const double sc = eps * l[i];
                 v[i] = make_double4(pm_start[3 * i] * sc, pm_start[3 * i + 1] * sc, pm_start[3 * i + 2] * sc, 0.0);
             }
-            ck(cudaMemcpy(pm_v, v.data(), N * sizeof(double4), cudaMemcpyHostToDevice), "upload");
+            h2d(pm_v, v.data(), N * sizeof(double4), "upload");
             pm_initialized = true;
         }
         const am::NodeDev nd = node_dev();
@@ -1594,7 +1602,7 @@ int am_create(int64_t num_nodes, const double* coords, am_ctx** out) {
         c->host_X.assign(coords, coords + 3 * N);
         std::vector<double4> x(N);
         for (size_t i = 0; i < N; ++i) x[i] = make_double4(coords[3 * i], coords[3 * i + 1], coords[3 * i + 2], 0.0);
-        ck(cudaMemcpy(c->X4, x.data(), N * sizeof(double4), cudaMemcpyHostToDevice), "coords upload");
+        h2d(c->X4, x.data(), N * sizeof(double4), "coords upload");
         ck(cudaMemset(c->U4, 0, N * sizeof(double4)), "memset");
         ck(cudaMemset(c->V4, 0, N * sizeof(double4)), "memset");
         ck(cudaMemset(c->A4, 0, N * sizeof(double4)), "memset");
@@ -1694,7 +1702,7 @@ int am_add_block(am_ctx* ctx, const am_block_desc* d, int32_t* block_id) {
                         b.num_patches = P;
                         b.slot_count = 8 * P;
                         b.patch_nodes = dalloc<int32_t>(8 * P, "patch nodes");
-                        ck(cudaMemcpy(b.patch_nodes, tp.nodes.data(), 8 * P * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
+                        h2d(b.patch_nodes, tp.nodes.data(), 8 * P * sizeof(int32_t), "upload");
                         b.host_nodes.assign(tp.nodes.begin(), tp.nodes.begin() + 8 * P);
                         ctx->upload_cell_units(b, d->cell_grads, d->cell_volumes);
                         if (ctx->warp_chunks && ctx->lagr == 0) {
@@ -1711,20 +1719,20 @@ int am_add_block(am_ctx* ctx, const am_block_desc* d, int32_t* block_id) {
                 }
                 if (b.patched == 0) {
                     b.cell_ptr = dalloc<int32_t>(E + 1, "cell ptr");
-                    ck(cudaMemcpy(b.cell_ptr, ptr.data(), (E + 1) * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
+                    h2d(b.cell_ptr, ptr.data(), (E + 1) * sizeof(int32_t), "upload");
                     if (K > 0) {
                         std::vector<float> g32(K * 3);
                         for (int64_t s = 0; s < K * 3; ++s) g32[s] = static_cast<float>(d->cell_grads[s]);
                         b.cell_nodes = dalloc<int32_t>(K, "cell nodes");
                         b.grads64 = dalloc<double>(K * 3, "cell grads");
                         b.grads32 = dalloc<float>(K * 3, "cell grads fp32");
-                        ck(cudaMemcpy(b.cell_nodes, d->cell_nodes, K * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
-                        ck(cudaMemcpy(b.grads64, d->cell_grads, K * 3 * sizeof(double), cudaMemcpyHostToDevice), "upload");
-                        ck(cudaMemcpy(b.grads32, g32.data(), K * 3 * sizeof(float), cudaMemcpyHostToDevice), "upload");
+                        h2d(b.cell_nodes, d->cell_nodes, K * sizeof(int32_t), "upload");
+                        h2d(b.grads64, d->cell_grads, K * 3 * sizeof(double), "upload");
+                        h2d(b.grads32, g32.data(), K * 3 * sizeof(float), "upload");
                     }
                     if (E > 0) {
                         b.volumes = dalloc<double>(E, "cell volumes");
-                        ck(cudaMemcpy(b.volumes, d->cell_volumes, E * sizeof(double), cudaMemcpyHostToDevice), "upload");
+                        h2d(b.volumes, d->cell_volumes, E * sizeof(double), "upload");
                     }
                 }
             } else {
@@ -1749,11 +1757,11 @@ int am_add_block(am_ctx* ctx, const am_block_desc* d, int32_t* block_id) {
                     conn = conn_ordered.data();
                     b.order = std::move(eo.order);
                     b.order_dev = dalloc<int32_t>(E, "element order");
-                    ck(cudaMemcpy(b.order_dev, b.order.data(), E * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
+                    h2d(b.order_dev, b.order.data(), E * sizeof(int32_t), "upload");
                 }
                 if (S > 0) {
                     b.conn = dalloc<int32_t>(S, "connectivity");
-                    ck(cudaMemcpy(b.conn, conn, S * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
+                    h2d(b.conn, conn, S * sizeof(int32_t), "upload");
                 }
                 b.host_nodes.assign(conn, conn + S);
                 if (d->kind == AM_TET4_GAUSS && E > 0 && ctx->tet4_patches && ctx->lagr == 0) {
@@ -1775,10 +1783,10 @@ int am_add_block(am_ctx* ctx, const am_block_desc* d, int32_t* block_id) {
                         b.patch_nodes = dalloc<int32_t>(8 * P, "patch nodes");
                         b.patch_local = dalloc<uint32_t>(E, "patch local ids");
                         b.patch_gather = dalloc<uint32_t>(8 * P, "patch gather masks");
-                        ck(cudaMemcpy(b.patch_gather, tp.gather.data(), 8 * P * sizeof(uint32_t), cudaMemcpyHostToDevice), "upload");
-                        ck(cudaMemcpy(b.patch_first, tp.first.data(), (P + 1) * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
-                        ck(cudaMemcpy(b.patch_nodes, tp.nodes.data(), 8 * P * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
-                        ck(cudaMemcpy(b.patch_local, tp.local.data(), E * sizeof(uint32_t), cudaMemcpyHostToDevice), "upload");
+                        h2d(b.patch_gather, tp.gather.data(), 8 * P * sizeof(uint32_t), "upload");
+                        h2d(b.patch_first, tp.first.data(), (P + 1) * sizeof(int32_t), "upload");
+                        h2d(b.patch_nodes, tp.nodes.data(), 8 * P * sizeof(int32_t), "upload");
+                        h2d(b.patch_local, tp.local.data(), E * sizeof(uint32_t), "upload");
                         if (hex6) {
                             b.patch_dx32 = dalloc<float>(21 * P, "patch coordinate differences");
                             b.patch_dx64 = dalloc<double>(21 * P, "patch coordinate differences");
@@ -1821,14 +1829,14 @@ int am_add_block(am_ctx* ctx, const am_block_desc* d, int32_t* block_id) {
                     if (!(d->mu_field[e] > 0.0)) fail(AM_EINVAL, "shear modulus field must be positive");
                 b.mu_field = dalloc<double>(E, "mu field");
                 const std::vector<double> v = b.to_order(d->mu_field);
-                ck(cudaMemcpy(b.mu_field, v.data(), E * sizeof(double), cudaMemcpyHostToDevice), "upload");
+                h2d(b.mu_field, v.data(), E * sizeof(double), "upload");
             }
             if (d->kappa_field && E > 0) {
                 for (int64_t e = 0; e < E; ++e)
                     if (!(d->kappa_field[e] > 0.0)) fail(AM_EINVAL, "bulk modulus field must be positive");
                 b.kappa_field = dalloc<double>(E, "kappa field");
                 const std::vector<double> v = b.to_order(d->kappa_field);
-                ck(cudaMemcpy(b.kappa_field, v.data(), E * sizeof(double), cudaMemcpyHostToDevice), "upload");
+                h2d(b.kappa_field, v.data(), E * sizeof(double), "upload");
             }
         } catch (...) {
             b.release();
@@ -1876,8 +1884,8 @@ int am_set_boundary_conditions(am_ctx* ctx, int32_t num_bcs, const am_bc_desc* b
             bc.nodes.assign(d.nodes, d.nodes + d.num_nodes);
             list.push_back(std::move(bc));
         }
-        ck(cudaMemcpy(ctx->bcword, word.data(), ctx->N * sizeof(uint32_t), cudaMemcpyHostToDevice), "bc upload");
-        ck(cudaMemcpy(ctx->bcvalues, values.data(), values.size() * sizeof(double), cudaMemcpyHostToDevice), "bc upload");
+        h2d(ctx->bcword, word.data(), ctx->N * sizeof(uint32_t), "bc upload");
+        h2d(ctx->bcvalues, values.data(), values.size() * sizeof(double), "bc upload");
         ctx->bcs = std::move(list);
     });
 }
@@ -1929,7 +1937,7 @@ int am_set_cell_groups(am_ctx* ctx, int32_t block_id, int64_t num_cells, const i
         const char* passes = std::getenv("APERI_B200_FBAR_PASSES");
         b.fbar_fused = !(passes && passes[0] == '3');
         b.group_ptr = dalloc<int64_t>(num_cells + 1, "cell groups");
-        ck(cudaMemcpy(b.group_ptr, group_ptr, (num_cells + 1) * sizeof(int64_t), cudaMemcpyHostToDevice), "upload");
+        h2d(b.group_ptr, group_ptr, (num_cells + 1) * sizeof(int64_t), "upload");
         if (!b.host_grads.empty()) b.host_group_ptr.assign(group_ptr, group_ptr + num_cells + 1);
     });
 }
@@ -1951,7 +1959,7 @@ int am_set_mass(am_ctx* ctx, const double* mass) {
         ctx->drop_graphs();
         for (int64_t i = 0; i < ctx->N; ++i)
             if (!(mass[i] > 0.0)) fail(AM_EINVAL, "nodal masses must be positive");
-        ck(cudaMemcpy(ctx->mass, mass, ctx->N * sizeof(double), cudaMemcpyHostToDevice), "mass upload");
+        h2d(ctx->mass, mass, ctx->N * sizeof(double), "mass upload");
         ctx->mass_set = true;
         ctx->mass_from_caller = true;
     });
@@ -1995,10 +2003,10 @@ int am_finalize(am_ctx* ctx) {
                 if (b.host_nodes[k] >= 0) pos[b.slot_base + k] = fill[b.host_nodes[k]]++;
         ctx->num_used_slots = ptr[NP];
         ctx->node_ptr = dalloc<int32_t>(NP + 1, "node ptr");
-        ck(cudaMemcpy(ctx->node_ptr, ptr.data(), (NP + 1) * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
+        h2d(ctx->node_ptr, ptr.data(), (NP + 1) * sizeof(int32_t), "upload");
         if (S > 0) {
             ctx->slot_pos = dalloc<int32_t>(S, "slot positions");
-            ck(cudaMemcpy(ctx->slot_pos, pos.data(), S * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
+            h2d(ctx->slot_pos, pos.data(), S * sizeof(int32_t), "upload");
             ctx->slots64 = dalloc<double4>(static_cast<size_t>(std::max<int64_t>(ctx->num_used_slots, 1)), "slot buffer");
         }
         for (auto& b : ctx->blocks) {
@@ -2046,7 +2054,7 @@ int am_finalize(am_ctx* ctx) {
                 m[i] = f[3 * i];
                 if (!(m[i] > 0.0)) fail(AM_EINVAL, "node " + std::to_string(i) + " has no mass (not connected to an element)");
             }
-            ck(cudaMemcpy(ctx->mass, m.data(), N * sizeof(double), cudaMemcpyHostToDevice), "mass upload");
+            h2d(ctx->mass, m.data(), N * sizeof(double), "mass upload");
             ctx->mass_set = true;
         }
         if (ctx->lagr) {
@@ -2172,7 +2180,7 @@ int am_set_power_method(am_ctx* ctx, const double* start, const double* max_edge
             ctx->pm_fe = dalloc<double>(3 * ctx->N, "force");
             ctx->pm_partial = dalloc<double>((ctx->N + 255) / 256, "partial sums");
         }
-        ck(cudaMemcpy(ctx->pm_l, max_edge_length, ctx->N * sizeof(double), cudaMemcpyHostToDevice), "upload");
+        h2d(ctx->pm_l, max_edge_length, ctx->N * sizeof(double), "upload");
         ctx->pm_initialized = false;
     });
 }
@@ -2399,7 +2407,7 @@ int am_stress(int32_t material, double lambda, double mu, int64_t n, am_memory w
             h1.reset(a);
             double* b = dalloc<double>(n * 9, "P");
             h2.reset(b);
-            ck(cudaMemcpy(a, H, n * 9 * sizeof(double), cudaMemcpyHostToDevice), "H2D");
+            h2d(a, H, n * 9 * sizeof(double), "H2D");
             dH = a;
             dP = b;
         }
@@ -2434,7 +2442,7 @@ int am_quadrature(int32_t kind, int32_t smoothed, int64_t n, am_memory where, co
             hold.emplace_back(b, [](double* p) { cudaFree(p); });
             double* c = dalloc<double>(nw, "w");
             hold.emplace_back(c, [](double* p) { cudaFree(p); });
-            ck(cudaMemcpy(a, X, nx * sizeof(double), cudaMemcpyHostToDevice), "H2D");
+            h2d(a, X, nx * sizeof(double), "H2D");
             dX = a;
             dB = b;
             dw = c;
@@ -2535,13 +2543,13 @@ int am_set_interface(am_ctx* ctx, int64_t num_local, const int32_t* local_nodes,
         ctx->iface_local = num_local;
         ctx->iface_global = num_global;
         ctx->iface_row_of = dalloc<int32_t>(ctx->N, "interface rows");
-        ck(cudaMemcpy(ctx->iface_row_of, row_of.data(), ctx->N * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
+        h2d(ctx->iface_row_of, row_of.data(), ctx->N * sizeof(int32_t), "upload");
         ctx->iface_buf = dalloc<double>(static_cast<size_t>(std::max<int64_t>(num_global, 1)) * 3, "interface buffer");
         if (num_local > 0) {
             ctx->iface_nodes = dalloc<int32_t>(num_local, "interface nodes");
             ctx->iface_rows = dalloc<int32_t>(num_local, "interface rows");
-            ck(cudaMemcpy(ctx->iface_nodes, local_nodes, num_local * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
-            ck(cudaMemcpy(ctx->iface_rows, rows, num_local * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
+            h2d(ctx->iface_nodes, local_nodes, num_local * sizeof(int32_t), "upload");
+            h2d(ctx->iface_rows, rows, num_local * sizeof(int32_t), "upload");
         }
     });
 }
@@ -2603,7 +2611,7 @@ int am_set_neighbors(am_ctx* ctx, int32_t rank, int32_t num_neighbors, const int
         ctx->iface_local = R;
         ctx->iface_global = R;
         ctx->iface_row_of = dalloc<int32_t>(ctx->N, "interface rows");
-        ck(cudaMemcpy(ctx->iface_row_of, row_of.data(), ctx->N * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
+        h2d(ctx->iface_row_of, row_of.data(), ctx->N * sizeof(int32_t), "upload");
         const size_t R1 = static_cast<size_t>(std::max<int64_t>(R, 1)), S1 = static_cast<size_t>(std::max<int64_t>(S, 1));
         ctx->iface_buf = dalloc<double>(R1 * 3, "interface buffer");
         ctx->nbr_own = dalloc<double>(R1 * 3, "interface partials");
@@ -2614,13 +2622,13 @@ int am_set_neighbors(am_ctx* ctx, int32_t rank, int32_t num_neighbors, const int
         ctx->comb_idx = dalloc<int32_t>(std::max<size_t>(cidx.size(), 1), "combine sources");
         ctx->iface_nodes = dalloc<int32_t>(R1, "interface nodes");
         ctx->iface_rows = dalloc<int32_t>(R1, "interface rows");
-        if (S > 0) ck(cudaMemcpy(ctx->nbr_send_rows, send_rows.data(), S * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
-        ck(cudaMemcpy(ctx->comb_ptr, cptr.data(), (R + 1) * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
+        if (S > 0) h2d(ctx->nbr_send_rows, send_rows.data(), S * sizeof(int32_t), "upload");
+        h2d(ctx->comb_ptr, cptr.data(), (R + 1) * sizeof(int32_t), "upload");
         if (!cidx.empty())
-            ck(cudaMemcpy(ctx->comb_idx, cidx.data(), cidx.size() * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
+            h2d(ctx->comb_idx, cidx.data(), cidx.size() * sizeof(int32_t), "upload");
         if (R > 0) {
-            ck(cudaMemcpy(ctx->iface_nodes, nodes.data(), R * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
-            ck(cudaMemcpy(ctx->iface_rows, rows.data(), R * sizeof(int32_t), cudaMemcpyHostToDevice), "upload");
+            h2d(ctx->iface_nodes, nodes.data(), R * sizeof(int32_t), "upload");
+            h2d(ctx->iface_rows, rows.data(), R * sizeof(int32_t), "upload");
         }
         const char* ov = std::getenv("APERI_B200_EXCHANGE_OVERLAP");
         ctx->overlap = !(ov && ov[0] == '0');
@@ -2701,7 +2709,7 @@ int am_set_rk_functions(am_ctx* ctx, const int64_t* nbr_ptr, const int32_t* nbr,
         auto up = [&](auto*& dst, const auto* src, int64_t n, const char* what) {
             using T0 = std::remove_reference_t<decltype(*dst)>;
             dst = dalloc<T0>(static_cast<size_t>(std::max<int64_t>(n, 1)), what);
-            if (n > 0) ck(cudaMemcpy(dst, src, n * sizeof(T0), cudaMemcpyHostToDevice), "upload");
+            if (n > 0) h2d(dst, src, n * sizeof(T0), "upload");
         };
         if (ctx->rk_octets) {
             // rows sorted by node and columns (ascending point already) in warp octets

@@ -13,7 +13,8 @@ mesh is one 70^3-hex z-slab per rank stacked into a 1 x 1 x N box, and every ste
 interface nodes' partial forces are summed across ranks with NCCL before the nodal
 update (weak scaling with the exchange the reference does with MPI).
 
-Prints one JSON line. `value` is the mixed FP32-element / FP64-state path in
+Prints one JSON line on stdout (the other workloads by their rates; their full records go to
+stderr as one JSON line). `value` is the mixed FP32-element / FP64-state path in
 Melem-steps/s (elements x steps / device seconds), with the plain FP64 path, the
 mixed-vs-FP64 errors, the adjoint/forward cost ratio (Hex8 neo-Hookean 64^3,
 200 steps, checkpoints every 20), the dominant kernel's roofline, an end-to-end
@@ -425,6 +426,7 @@ def measure_workload(torch, prob, steps, warmup, stream, dev, world, mass=None, 
     if formulation is not None:
         out["formulation"] = list(formulation)
     peak, kind = measured_peaks()
+    name = prob.name if formulation is None else None  # the captures are of the total formulation
     with ExplicitDynamics(prob.coords, prob.parts, prob.bcs, mass=mass, stream=stream.cuda_stream,
                           rk=prob.meta.get("rk"), formulation=formulation) as m:
         layout = m.layout()
@@ -443,10 +445,10 @@ def measure_workload(torch, prob, steps, warmup, stream, dev, world, mass=None, 
             out["mixed_rel_force_err_l2"] = err["rel_force_err_l2"]
         if "mixed" in precs:
             out["roofline_mixed"] = roofline_for(out["mixed"]["kernels"], algorithmic_bytes(prob, layout), peak, kind,
-                                                 prob.name, "mixed", algorithmic_flop(prob), fma)
+                                                 name, "mixed", algorithmic_flop(prob), fma)
         if "fp64" in precs:
             out["roofline_fp64"] = roofline_for(out["fp64"]["kernels"], algorithmic_bytes(prob, layout, 24), peak, kind,
-                                                prob.name, "fp64", algorithmic_flop(prob), fma)
+                                                name, "fp64", algorithmic_flop(prob), fma)
     return out
 
 
@@ -744,6 +746,16 @@ def run_reference(args, rank, world):
     print(json.dumps(line), flush=True)
 
 
+def brief(record):
+    """A workload's rates and mixed error, for the printed line."""
+    out = {p: round(record[p]["value"], 1) for p in ("fp64", "mixed") if p in record}
+    if "mixed_rel_disp_err_l2" in record:
+        out["mixed_err"] = float(f"{record['mixed_rel_disp_err_l2']:.2e}")
+    if "adjoint" in record:
+        out["adjoint_ratio"] = round(record["adjoint"]["ratio"], 3)
+    return out
+
+
 def main():
     args = parse()
     rank, world, local = dist_init(args.gpus)
@@ -773,8 +785,9 @@ def main():
         "e2e": e2e,
         "gpu_launches": launches["mixed"],
         "clocks": clocks,
-        "other_workloads": extras,
+        "other_workloads": {name: brief(r) for name, r in extras.items()},
     }
+    print(json.dumps({"other_workloads": extras}), file=sys.stderr, flush=True)
     print(json.dumps(line), flush=True)
 
 

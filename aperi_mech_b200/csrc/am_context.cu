@@ -1816,8 +1816,9 @@ int am_add_block(am_ctx* ctx, const am_block_desc* d, int32_t* block_id) {
                     am::launch_tet4_geometry(b.conn, E, ctx->X4, b.geo32, b.geo64, ctx->stream);
                     ck(cudaGetLastError(), "tet geometry");
                 }
-                // Warp chunks for the one-thread-per-tet kernels (Hex8 measured no gain: its
-                // issue-bound element kernel paid for the warp sums what its node kernel saved).
+                // Warp chunks for the one-thread-per-tet kernels. Hex8 measured no gain with one
+                // thread per element, FP64 and mixed (its element kernel paid for the warp sums
+                // what its node kernel saved); with the FP64 quads it was not measured.
                 WarpChunks wc;
                 if (ctx->warp_chunks && E > 0 && d->kind == AM_TET4_GAUSS && (b.geo64 || ctx->lagr != 0) &&
                     build_warp_chunks(conn, E, nn, wc))

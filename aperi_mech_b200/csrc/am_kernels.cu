@@ -1327,7 +1327,8 @@ __device__ __forceinline__ void lagr_pull(const double* hr, const double* P, dou
 // one wait covers both. Latency of those loads binds (FP64 pipe 36%), hence 20 warps per SM
 // for a few spilled registers. On a 45 x 45 x 61 box (741,150 tets, B200, 1965 MHz, semi with
 // an update every 10 steps), us per step: four slots per tet and H written every step 79.8;
-// chunks and keep 60.4; H_ref first 55.3; 20 warps 51.4 (24 warps, more spills: 52.3).
+// chunks and keep 60.4; H_ref first 55.3; 20 warps 51.4 (24 warps, more spills: 52.3); the
+// H arrays padded, 50.2.
 template <int MAT, bool CHUNKS>
 __global__ void __launch_bounds__(128, 5) k_tet4_force_lagr(GaussBlockDev b, int32_t lagr, int rebase, int keep,
                                                           const double4* __restrict__ XC,

@@ -930,8 +930,9 @@ __device__ __forceinline__ void hex_conn(const GaussBlockDev& b, int64_t e, int3
 // point's tensors: 246 registers and eight warps per SM, and 250 warps in all on 8,000
 // elements. A quad's lane needs 128 registers and a quarter of the serial work. Measured on
 // B200 (1965 MHz), one thread per element against this kernel: a step of 20^3 linear elastic
-// 10.8 -> 7.7 us; 128^3 neo-Hookean with fields, per launch, 523 -> 459 us. The FP64 pipe is
-// 53% busy (its floor is 290 us at 128^3), gather latency takes the rest.
+// 10.8 -> 7.7 us; 128^3 neo-Hookean with fields, per launch, 523 -> 459 us (423 with the
+// connectivity past L1). The FP64 pipe is 62% busy, the L1 wavefronts 63%; gather latency
+// takes the rest.
 // ---------------------------------------------------------------------------
 constexpr double kHexR = 0.26794919243112270647;   // (1 - c) / (1 + c) = 2 - sqrt 3
 constexpr double kHexScale = 0.31100423396407310780;  // (1 + c)^2 / 8: derivative = kHexScale x raw
@@ -1324,7 +1325,7 @@ __device__ __forceinline__ void lagr_pull(const double* hr, const double* P, dou
 // k_tet4_force_geo. keep: this evaluation's H may become a reference gradient (every step
 // under the updated formulation, the last step before a reference update under the semi
 // one); otherwise it is not written. A tet reads its H_ref before its gathers, so that the
-// one wait covers both. Latency of those loads binds (FP64 pipe 36%), hence 20 warps per SM
+// one wait covers both. Latency of those loads binds (FP64 pipe 44%), hence 20 warps per SM
 // for a few spilled registers. On a 45 x 45 x 61 box (741,150 tets, B200, 1965 MHz, semi with
 // an update every 10 steps), us per step: four slots per tet and H written every step 79.8;
 // chunks and keep 60.4; H_ref first 55.3; 20 warps 51.4 (24 warps, more spills: 52.3); the
@@ -1943,8 +1944,8 @@ __global__ void __launch_bounds__(256) k_cell_units(const double* __restrict__ g
 
 // Gradients and volumes come from the half-patch tables, whose vec4 loads are contiguous over
 // a warp (from the cells' own rows a lane's loads lay 144 bytes apart): h = 1/46 box mixed
-// 35.3 -> 33.0 us a step, and 30.6 with the tables kept out of L1. Bound: 97 MB of tables,
-// plans and slots at 55% of the measured HBM rate, latency of the u gathers.
+// 35.3 -> 33.0 us a step, and 30.6 with the tables kept out of L1. Bound: latency of the u
+// gathers; the compulsory bytes move at 50% of the measured HBM rate (88 MB of traffic).
 template <typename T, int MAT, bool CHUNKS>
 __global__ void __launch_bounds__(kHex6Block, hex6_min_blocks<T>()) k_cell_hex6_force(CellBlockDev b, const double4* U4,
                                                                                     vec4_t<T>* slots, int* status) {
